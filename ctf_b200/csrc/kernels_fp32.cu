@@ -1,11 +1,16 @@
 // FP32-bulk step kernels: reconstruction, Riemann fluxes and the RK combine of the five
 // hydrodynamic components in FP32; the magnetic field, its constrained-transport update, the
 // c2p Newton polish and the dt reduction in FP64.
-// the flux sweep at 4 resident blocks of 128 threads per SM (chosen by a sweep of 1-4)
+// the HLL and HLLC sweeps at 4 resident blocks of 128 threads per SM (chosen by a sweep of 1-4)
 #ifdef MGPU_FLUX_MINB_OVERRIDE
 #define MGPU_FLUX_MINB MGPU_FLUX_MINB_OVERRIDE
 #else
 #define MGPU_FLUX_MINB 4
+#endif
+// HLLD sweeps (rmhd_face32.cuh) at 6 blocks, 80 registers: 160^3 lean sweeps per RK3 step 3.82 /
+// 3.34 / 3.29 ms (PLM) and 5.80 / 4.86 / 4.75 ms (WENO5) at 4 / 5 / 6 blocks
+#ifndef MGPU_HLLD_MINB
+#define MGPU_HLLD_MINB 6
 #endif
 #ifdef MGPU_C2P_MINB_OVERRIDE
 #define MGPU_C2P_MINB MGPU_C2P_MINB_OVERRIDE

@@ -71,7 +71,18 @@ __device__ __forceinline__ int ctu_riemann(const PhysParams &pp, const T *Pl, co
   if constexpr (RS == RIEMANN_HLLD) {
     C2PTally t{0, 0};
     int used_hllc = 0;
-    err = riemann_hlld<T, dim>(pp, Pl, Pr, Fo, ml, used_hllc, &t);
+    if constexpr (sizeof(T) < sizeof(double)) {
+      const auto src = [&](float *l, float *r) {
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          l[q] = Pl[q];
+          r[q] = Pr[q];
+        }
+      };
+      err = riemann_hlld32<dim>(pp, Pl, Pr, Fo, ml, used_hllc, &t, src);
+    } else {
+      err = riemann_hlld<T, dim>(pp, Pl, Pr, Fo, ml, used_hllc, &t);
+    }
     ft.hlld_ok += 1 - used_hllc;
     ft.hlld_hllc += used_hllc;
     ft.face_c2p_calls += t.attempts > 0;
@@ -87,7 +98,7 @@ __device__ __forceinline__ int ctu_riemann(const PhysParams &pp, const T *Pl, co
 // Both flux passes of one direction (dim 1..3); pass 1 reads its states from PA, pass 2 from
 // the predicted primitives Pd of this direction.  One thread per face.
 template <class T, int dim, int RS>
-__global__ void __launch_bounds__(128, MGPU_FLUX_MINB) k_ctu_flux(Grid g, const T *__restrict__ PA,
+__global__ void __launch_bounds__(128, flux_minb<RS>()) k_ctu_flux(Grid g, const T *__restrict__ PA,
                                                                   const T *__restrict__ Pd, T *__restrict__ F,
                                                                   PhysParams pp, Ctl *ctl, int stage, int pass)
 {

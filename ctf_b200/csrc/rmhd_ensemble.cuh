@@ -106,7 +106,7 @@ __global__ void __launch_bounds__(128) k_ens_c2p(const BoxDev *boxes, const int2
 }
 
 template <class T, int dim, int RS>
-__global__ void __launch_bounds__(128, MGPU_FLUX_MINB) k_ens_flux(const BoxDev *boxes, const int2 *map,
+__global__ void __launch_bounds__(128, flux_minb<RS>()) k_ens_flux(const BoxDev *boxes, const int2 *map,
                                                                   long long ntiles, int tile, PhysParams pp,
                                                                   int stage)
 {

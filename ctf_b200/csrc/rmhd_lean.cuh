@@ -83,11 +83,13 @@ __device__ __forceinline__ void lean_accumulate(const Grid &g, StatePtr<T> U0, S
 // ---- x and y sweeps: one thread per (column, chunk), marching along the sweep direction ---------
 // Columns cover the two other dimensions with one zone of halo ([ng-1, ng+n] each: flux-CT
 // reads transverse neighbours' face fields); a chunk is `chunk` zones of the sweep direction
-// (lean_chunk picks it per launch).  The thread computes the lower face of its first zone, then per zone the upper
-// face, and adds the difference to the zone when the column is interior.  Consecutive threads
-// take consecutive k, so every load and store is coalesced.
+// (lean_chunk picks it per launch).  The thread computes the lower face of its first zone, then
+// per zone the upper face, and adds the difference to the zone when the column is interior.
+// Each zone is reconstructed once, both its faces together: the upper face value waits in
+// shared memory for the next face.  Consecutive threads take consecutive k, so every load and
+// store is coalesced.
 template <class T, int dim, int RS>
-__global__ void __launch_bounds__(128, MGPU_FLUX_MINB) k_lean_sweep(Grid g, const T *__restrict__ PA, StatePtr<T> UA,
+__global__ void __launch_bounds__(128, flux_minb<RS>()) k_lean_sweep(Grid g, const T *__restrict__ PA, StatePtr<T> UA,
                                                                     StatePtr<T> UB, T *__restrict__ Bf,
                                                                     LeanCombine c, PhysParams pp, Ctl *ctl, int stage,
                                                                     int chunk_len)
@@ -110,7 +112,7 @@ __global__ void __launch_bounds__(128, MGPU_FLUX_MINB) k_lean_sweep(Grid g, cons
   T ml = T(0);
   FluxTally ft{0, 0, 0, 0, 0};
   __shared__ T flo[128][5];   // the carried lower-face flux of each thread
-  __shared__ HlldSlot<T> hslot[RS == RIEMANN_HLLD && sizeof(T) < sizeof(double) ? 128 : 1];
+  __shared__ T up[8][128];    // the carried upper-face state of the face's lower zone
   if (t < ncol * nchunk) {
     const int chunk = (int) (t / ncol);
     const long long col = t - (long long) chunk * ncol;
@@ -126,6 +128,12 @@ __global__ void __launch_bounds__(128, MGPU_FLUX_MINB) k_lean_sweep(Grid g, cons
     const T dt = T(ctl->dt);
     T *slot0 = Bf + (long long) bf_slot(dim, dim == 1 ? By : Bx) * g.cs;
     T *slot1 = Bf + (long long) bf_slot(dim, Bz) * g.cs;
+    {
+      T lo[8], hi[8];
+      zone_states<T>(PA, g.cs, S, pp, base + (long long) (m0 - 1) * S, lo, hi);
+#pragma unroll
+      for (int q = 0; q < 8; ++q) up[q][threadIdx.x] = hi[q];
+    }
 #pragma unroll 1
     for (int m = m0 - 1; m < m1; ++m) {   // face between zones m and m + 1
       const long long f = base + (long long) m * S;
@@ -136,9 +144,13 @@ __global__ void __launch_bounds__(128, MGPU_FLUX_MINB) k_lean_sweep(Grid g, cons
           if (dim == 1) asm volatile("prefetch.global.L2 [%0];" ::"l"(U0.bulk + q * g.cs + f));
         }
       }
-      T Fo[8];
-      face_flux<T, dim, RS>(g, PA, pp, f, ml, ft, Fo,
-                            RS == RIEMANN_HLLD && sizeof(T) < sizeof(double) ? &hslot[threadIdx.x] : nullptr);
+      T Pl[8], Pr[8], hi[8], Fo[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) Pl[q] = up[q][threadIdx.x];
+      zone_states<T>(PA, g.cs, S, pp, f + S, Pr, hi);
+#pragma unroll
+      for (int q = 0; q < 8; ++q) up[q][threadIdx.x] = hi[q];
+      solve_face<T, dim, RS>(g, PA, pp, f, Pl, Pr, ml, ft, Fo);
       if (m >= m0 || chunk == 0) {            // the chunk's first face is its neighbour's last
         slot0[f] = Fo[dim == 1 ? By : Bx];
         slot1[f] = Fo[Bz];
@@ -151,12 +163,14 @@ __global__ void __launch_bounds__(128, MGPU_FLUX_MINB) k_lean_sweep(Grid g, cons
   flux_block_finish(double(ml), ft, ctl, RS == RIEMANN_HLLD);
 }
 
-// ---- z sweep (contiguous direction): 128 consecutive faces per CTA, shared-memory pairing ------
-// Rows are (i, j) with one zone of halo; a row holds the n2 + 1 faces [ng-1, ng+n2-1].  The
-// faces of all rows are numbered consecutively; CTA c computes faces 127 c - 1 .. 127 c + 126
-// and updates the zones whose both faces it holds (its first face is the previous CTA's last).
+// ---- z sweep (contiguous direction): 128 consecutive zones per CTA, shared-memory pairing ------
+// Rows are (i, j) with one zone of halo; a row holds the n2 + 2 zones [ng-1, ng+n2].  The zones
+// of all rows are numbered consecutively.  Thread t of CTA c reconstructs zone 126 c - 2 + t
+// (both its faces), solves the face below it with the upper state of thread t - 1's zone, and
+// from the fluxes of threads t - 1 and t updates the zone below it; so each CTA solves 127
+// faces and updates 126 zones, its first face being the previous CTA's last.
 template <class T, int RS>
-__global__ void __launch_bounds__(128, MGPU_FLUX_MINB) k_lean_sweep_z(Grid g, const T *__restrict__ PA, StatePtr<T> UA,
+__global__ void __launch_bounds__(128, flux_minb<RS>()) k_lean_sweep_z(Grid g, const T *__restrict__ PA, StatePtr<T> UA,
                                                                       StatePtr<T> UB, T *__restrict__ Bf,
                                                                       LeanCombine c, PhysParams pp, Ctl *ctl,
                                                                       int stage)
@@ -164,37 +178,48 @@ __global__ void __launch_bounds__(128, MGPU_FLUX_MINB) k_lean_sweep_z(Grid g, co
   if (stage_failed(ctl, stage + 1)) return;
   StatePtr<T> U0, U1;
   lean_regs(ctl, UA, UB, U0, U1);
-  const int nf = g.n[2] + 1, nj = g.n[1] + 2;
+  const unsigned nr = g.n[2] + 2, nj = g.n[1] + 2;
   // the window's x rows and the halo rows it computes: a - 1 in [win_flo, win_fhi)
   const int alo = win_lo(g), ahi = win_hi(g), a0 = win_flo(g) + 1;
-  const long long total = (long long) (win_fhi(g) - win_flo(g)) * nj * nf;
-  const long long q = (long long) blockIdx.x * 127 - 1 + threadIdx.x;
+  const unsigned total = (unsigned) (win_fhi(g) - win_flo(g)) * nj * nr;   // < 2^31: the grid is 1-D
+  const int q = (int) (blockIdx.x * 126u) - 2 + (int) threadIdx.x;
   T ml = T(0);
   FluxTally ft{0, 0, 0, 0, 0};
-  __shared__ T fs[5][128];
-  __shared__ HlldSlot<T> hslot[RS == RIEMANN_HLLD && sizeof(T) < sizeof(double) ? 128 : 1];
-  const bool active = q >= 0 && q < total;
-  long long f = 0;
-  bool upd = false;
-  if (active) {
-    const long long row = q / nf;
-    const int fk = (int) (q - row * nf);              // face fk + ng - 1
-    const int ar = (int) (row / nj), b = (int) (row - (long long) ar * nj);
-    const int a = a0 + ar;
-    const int i = g.ng - 1 + a, j = g.ng - 1 + b;
-    f = (long long) i * g.s[0] + (long long) j * g.s[1] + (g.ng - 1 + fk);
+  __shared__ T up[8][128];   // each zone's upper state
+  __shared__ T fs[5][128];   // each thread's flux
+  T Pl[8], Pr[8];
+  long long z = 0;
+  int fk = 0;
+  bool face = false, upd = false;
+  if (q >= 0 && (unsigned) q < total) {
+    const unsigned row = (unsigned) q / nr;
+    fk = (int) ((unsigned) q - row * nr);              // zone fk + ng - 1, its lower face
+    const unsigned ar = row / nj;
+    const int b = (int) (row - ar * nj), a = a0 + (int) ar;
+    z = (long long) (g.ng - 1 + a) * g.s[0] + (long long) (g.ng - 1 + b) * g.s[1] + (g.ng - 1 + fk);
+    face = threadIdx.x > 0 && fk >= 1;
+    upd = threadIdx.x > 1 && fk >= 2 && a >= alo + 1 && a <= ahi && b >= 1 && b <= g.n[1];
+    if (upd) {
 #pragma unroll
-    for (int r = 0; r < 5; ++r) asm volatile("prefetch.global.L2 [%0];" ::"l"(U1.bulk + r * g.cs + f));
+      for (int r = 0; r < 5; ++r) asm volatile("prefetch.global.L2 [%0];" ::"l"(U1.bulk + r * g.cs + z - 1));
+    }
+    T hi[8];
+    zone_states<T>(PA, g.cs, 1, pp, z, Pr, hi);
+#pragma unroll
+    for (int r = 0; r < 8; ++r) up[r][threadIdx.x] = hi[r];
+  }
+  __syncthreads();
+  if (face) {
     T Fo[8];
-    face_flux<T, 3, RS>(g, PA, pp, f, ml, ft, Fo,
-                        RS == RIEMANN_HLLD && sizeof(T) < sizeof(double) ? &hslot[threadIdx.x] : nullptr);
-    if (threadIdx.x > 0 || blockIdx.x == 0) {
-      Bf[(long long) bf_slot(3, Bx) * g.cs + f] = Fo[Bx];
-      Bf[(long long) bf_slot(3, By) * g.cs + f] = Fo[By];
+#pragma unroll
+    for (int r = 0; r < 8; ++r) Pl[r] = up[r][threadIdx.x - 1];
+    solve_face<T, 3, RS>(g, PA, pp, z - 1, Pl, Pr, ml, ft, Fo);
+    if (threadIdx.x > 1 || blockIdx.x == 0) {
+      Bf[(long long) bf_slot(3, Bx) * g.cs + z - 1] = Fo[Bx];
+      Bf[(long long) bf_slot(3, By) * g.cs + z - 1] = Fo[By];
     }
 #pragma unroll
     for (int r = 0; r < 5; ++r) fs[r][threadIdx.x] = Fo[r];
-    upd = threadIdx.x > 0 && fk >= 1 && a >= alo + 1 && a <= ahi && b >= 1 && b <= g.n[1];
   }
   __syncthreads();
   if (upd) {
@@ -204,7 +229,7 @@ __global__ void __launch_bounds__(128, MGPU_FLUX_MINB) k_lean_sweep_z(Grid g, co
       lo[r] = fs[r][threadIdx.x - 1];
       hi[r] = fs[r][threadIdx.x];
     }
-    lean_accumulate<T>(g, U0, U1, f, lo, hi, T(1.0 / g.dz), c, T(ctl->dt), false);
+    lean_accumulate<T>(g, U0, U1, z - 1, lo, hi, T(1.0 / g.dz), c, T(ctl->dt), false);
   }
   flux_block_finish(double(ml), ft, ctl, RS == RIEMANN_HLLD);
 }
@@ -364,8 +389,8 @@ inline void launch_lean_sweep(const Grid &g, int dim, int rs, cudaStream_t st, c
 {
   const unsigned blk = 128;
   if (dim == 3) {
-    const long long total = (long long) (win_fhi(g) - win_flo(g)) * (g.n[1] + 2) * (g.n[2] + 1);
-    const unsigned grid = (unsigned) ((total + 126) / 127);
+    const long long total = (long long) (win_fhi(g) - win_flo(g)) * (g.n[1] + 2) * (g.n[2] + 2);
+    const unsigned grid = (unsigned) ((total + 125) / 126);
 #define MGPU_LEANZ_CASE(R) \
   if (rs == R) { k_lean_sweep_z<T, R><<<grid, blk, 0, st>>>(g, PA, UA, UB, Bf, c, pp, ctl, s); return; }
     MGPU_LEANZ_CASE(RIEMANN_HLLD) MGPU_LEANZ_CASE(RIEMANN_HLLC) MGPU_LEANZ_CASE(RIEMANN_HLL)
@@ -377,7 +402,7 @@ inline void launch_lean_sweep(const Grid &g, int dim, int rs, cudaStream_t st, c
   const long long ncol = dim == 1 ? (long long) (g.n[1] + 2) * (g.n[2] + 2)
                                   : (long long) (win_fhi(g) - win_flo(g)) * (g.n[2] + 2);
   const int nmarch = dim == 1 ? win_rows(g) : g.n[1];
-  const int L = lean_chunk(ncol, nmarch, 148ll * MGPU_FLUX_MINB * blk);
+  const int L = lean_chunk(ncol, nmarch, 148ll * (rs == RIEMANN_HLLD ? flux_minb<RIEMANN_HLLD>() : flux_minb<RIEMANN_HLLC>()) * blk);
   const long long nchunk = (nmarch + L - 1) / L;
   const unsigned grid = (unsigned) ((ncol * nchunk + blk - 1) / blk);
 #define MGPU_LEAN_CASE(D, R) \

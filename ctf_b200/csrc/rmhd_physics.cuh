@@ -156,13 +156,8 @@ __device__ __forceinline__ void cubic(T c2, T c1, T c0, T &x1, T &x2, T &x3, int
 
 // Returns (max root, min root) over the real roots of d4 x^4 + ... + d0 with the fold used
 // by FluxAndEigenvalues: start at (-1, +1), then clamp to (1, -1) if either exceeds 1.
-// MGPU_QUARTIC_INLINE: inlined at every call site (the default), or __noinline__ for one
-// shared copy (less code in the long HLLD kernels).
-#ifndef MGPU_QUARTIC_INLINE
-#define MGPU_QUARTIC_INLINE __forceinline__
-#endif
 template <class T>
-__device__ MGPU_QUARTIC_INLINE void quartic_extreme_roots(T d4, T d3, T d2, T d1, T d0, T &ap, T &am)
+__device__ __forceinline__ void quartic_extreme_roots(T d4, T d3, T d2, T d1, T d0, T &ap, T &am)
 {
   const T a3 = d3 / d4, a2 = d2 / d4, a1 = d1 / d4, a0 = d0 / d4;
   const T au2 = -a2;
@@ -210,6 +205,79 @@ __device__ MGPU_QUARTIC_INLINE void quartic_extreme_roots(T d4, T d3, T d2, T d1
     ap = T(1);
     am = T(-1);
   }
+}
+
+// ---- fast magnetosonic speeds, FP32 --------------------------------------------------------------
+// The quartic of Mara/rmhd.cpp:275-305 divided by rho h W^2 and written in d = lambda - v:
+//   c4 d^4 + c3 d^3 + c2 d^2 + c1 d + c0.
+// In this form nothing cancels (the expanded coefficients lose all their digits near
+// degenerate roots and at high W, where FP32 Ferrari left errors of order one in the speed).
+// r0, r1: the speeds at zero normal field, outside the fast roots.
+struct FastQuartic {
+  float c4, c3, c2, c1, c0, hi, lo;
+};
+
+__device__ __forceinline__ FastQuartic fast_quartic(float gamma, float p, float rh, float b2, float W2, float iW2,
+                                                    float v, float vB, float B1)
+{
+  FastQuartic q;
+  const float irh = 1.f / rh, ics2 = rh / (gamma * p);
+  const float M = W2 * (ics2 - 1.f), L = 1.f + b2 * irh * ics2;
+  const float w = B1 * iW2;
+  const float uu = vB * vB * irh, uw = vB * w * irh, ww = w * w * irh;
+  const float g0 = 1.f - v * v;
+  q.c4 = M + L - uu;
+  q.c3 = 2.f * (v * (L - uu) + uw);
+  q.c2 = g0 * (uu - L) + 4.f * v * uw - ww;
+  q.c1 = -2.f * (v * ww + uw * g0);
+  q.c0 = ww * g0;
+  const float r = sqrtf(L * (L + M * g0)), is = 1.f / (M + L);
+  q.hi = (r - L * v) * is;
+  q.lo = (-r - L * v) * is;
+  return q;
+}
+
+// One Laguerre step toward the extreme root on side sg (+1 the largest, -1 the smallest): cubic
+// convergence, monotone from outside since the quartic's roots are real.
+__device__ __forceinline__ float laguerre_step(const FastQuartic &q, float d, float sg)
+{
+  float f = q.c4, f1 = q.c4, f2 = q.c4;
+  f = f * d + q.c3; f1 = f1 * d + f; f2 = f2 * d + f1;
+  f = f * d + q.c2; f1 = f1 * d + f; f2 = f2 * d + f1;
+  f = f * d + q.c1; f1 = f1 * d + f;
+  f = f * d + q.c0;
+  const float D = fmaxf(9.f * f1 * f1 - 24.f * f * f2, 0.f);
+  return 4.f * f / (f1 + sg * sqrtf(D));
+}
+
+// Both extreme roots from the given starts.  A step of s leaves an error of order s^3, so the
+// step below 5e-4 is the last one.
+__device__ __forceinline__ void laguerre_pair(const FastQuartic &q, float &hi, float &lo)
+{
+#pragma unroll 1
+  for (int it = 0; it < 8; ++it) {
+    const float a = laguerre_step(q, hi, 1.f), b = laguerre_step(q, lo, -1.f);
+    hi -= a;
+    lo -= b;
+    if (!(fmaxf(fabsf(a), fabsf(b)) > 5e-4f)) break;
+  }
+}
+
+// The speeds of a state outside the fluid's range (p <= 0 or rho <= 0, which reconstruction can
+// produce and P->U accepts): the reference's closed form on the expanded coefficients.
+static __device__ __noinline__ float2 irregular_speeds(float gamma, float r, float p, float v, float W2, float b0,
+                                                       float b2, float bi)
+{
+  const float h = 1.f + p / (gamma - 1.f) / r + p / r;
+  const float cs2 = eos_cs2(gamma, r, p);
+  const float W4 = W2 * W2, v2 = v * v, v3 = v * v2, v4 = v * v3;
+  const float K = r * h * (1.f / cs2 - 1.f) * W4;
+  const float L = -(r * h + b2 / cs2) * W2;
+  float2 o;
+  quartic_extreme_roots<float>(K - L - b0 * b0, -4.f * K * v + L * v * 2.f + 2.f * b0 * bi,
+                               6.f * K * v2 + L * (1.f - v2) + b0 * b0 - bi * bi,
+                               -4.f * K * v3 - L * v * 2.f - 2.f * b0 * bi, K * v4 + L * v2 + bi * bi, o.x, o.y);
+  return o;
 }
 
 // ---- flux and fast speeds (Mara/rmhd.cpp:208-310) ---------------------------------------
@@ -267,6 +335,26 @@ __device__ __forceinline__ void flux_and_eigenvalues(T gamma, const T *U, const 
     bi = bz;
   }
   if (!want_speeds) return;
+  if constexpr (sizeof(T) < sizeof(double)) {
+    if (P[pre] > T(0) && P[rho] > T(0)) {
+      const FastQuartic q = fast_quartic(gamma, P[pre], P[rho] * h, b2, W2, T(1) - V2, vi, Bv,
+                                         dim == 1 ? P[Bx] : dim == 2 ? P[By] : P[Bz]);
+      ap = q.hi;
+      am = q.lo;
+      laguerre_pair(q, ap, am);
+      ap += vi;
+      am += vi;
+      if (!(ap <= T(1) && am >= T(-1))) {
+        ap = T(1);
+        am = T(-1);
+      }
+    } else {
+      const float2 o = irregular_speeds(gamma, P[rho], P[pre], vi, W2, b0, b2, bi);
+      ap = o.x;
+      am = o.y;
+    }
+    return;
+  }
   const T cs2 = eos_cs2(gamma, P[rho], P[pre]);
   const T W4 = W2 * W2, v2 = vi * vi, v3 = vi * v2, v4 = vi * v3;
   const T K = P[rho] * h * (T(1) / cs2 - T(1)) * W4;
@@ -608,22 +696,74 @@ __device__ __forceinline__ T max3(T a, T b, T c)
   return x01 > c ? x01 : c;
 }
 
+// minmod of three slopes, as the reference's 0.25 |sgn a + sgn b| (sgn a + sgn c) min(|a|, |b|, |c|):
+// the common sign times the smallest magnitude, or zero.  In FP32 by minima and maxima (six
+// operations without the integer signs and their conversions; the same value for every
+// triple of numbers).
+template <class T>
+__device__ __forceinline__ T minmod3(T a, T b, T c)
+{
+  if constexpr (sizeof(T) < sizeof(double)) {
+    return fmaxf(fminf(fminf(a, b), c), 0.f) + fminf(fmaxf(fmaxf(a, b), c), 0.f);
+  } else {
+    const int sa = sgn(a), sb = sgn(b), sc = sgn(c);
+    return T(0.25) * T(abs(sa + sb)) * T(sa + sc) * min3(m_abs(a), m_abs(b), m_abs(c));
+  }
+}
+
 // PLM minmod(theta): face value v0 + sgn * slope / 2
 template <class T>
 __device__ __forceinline__ T plm(T theta, T vm, T v0, T vp, T sg)
 {
-  const T a = theta * (v0 - vm);
-  const T b = T(0.5) * (vp - vm);
-  const T c = theta * (vp - v0);
-  const int sa = sgn(a), sb = sgn(b), sc = sgn(c);
-  const T mm = T(0.25) * T(abs(sa + sb)) * T(sa + sc) * min3(m_abs(a), m_abs(b), m_abs(c));
-  return v0 + sg * T(0.5) * mm;
+  return v0 + sg * T(0.5) * minmod3(theta * (v0 - vm), T(0.5) * (vp - vm), theta * (vp - v0));
 }
 
-// WENO5 finite-volume, centre-to-right (c2r = true) or centre-to-left face, on the stencil
-// v[-2..2] given as (vm2, vm1, v0, vp1, vp2).
+// Both face values of the zone v0: toward vm (lo) and toward vp (hi), each as plm gives it.
 template <class T>
-__device__ __forceinline__ T weno5(int is_mode, T sz10A, T vm2, T vm1, T v0, T vp1, T vp2, bool c2r)
+__device__ __forceinline__ void plm_zone(T theta, T vm, T v0, T vp, T &lo, T &hi)
+{
+  const T h = T(0.5) * minmod3(theta * (v0 - vm), T(0.5) * (vp - vm), theta * (vp - v0));
+  lo = v0 - h;
+  hi = v0 + h;
+}
+
+// WENO5 smoothness indicators of the stencil v[-2..2], the same for both faces of the zone: for
+// JS96 and SZ10 the squared denominators of the weights, for B08 the factors 1 + tau5 / (B + eps).
+template <class T>
+__device__ __forceinline__ void weno5_indicators(int is_mode, T sz10A, T vm2, T vm1, T v0, T vp1, T vp2, T *k)
+{
+  const T t0a = T(1) * v0 - T(2) * vp1 + T(1) * vp2, t0b = T(3) * v0 - T(4) * vp1 + T(1) * vp2;
+  const T t1a = T(1) * vm1 - T(2) * v0 + T(1) * vp1, t1b = T(1) * vm1 - T(0) * v0 - T(1) * vp1;
+  const T t2a = T(1) * vm2 - T(2) * vm1 + T(1) * v0, t2b = T(1) * vm2 - T(4) * vm1 + T(3) * v0;
+  T B0 = T(13. / 12.) * (t0a * t0a) + T(1. / 4.) * (t0b * t0b);
+  T B1 = T(13. / 12.) * (t1a * t1a) + T(1. / 4.) * (t1b * t1b);
+  T B2 = T(13. / 12.) * (t2a * t2a) + T(1. / 4.) * (t2b * t2b);
+  if (is_mode == IS_B08) {
+    const T eps = T(1e-14);
+    const T tau5 = m_abs(B0 - B2);
+    k[0] = T(1) + (tau5 / (B0 + eps));
+    k[1] = T(1) + (tau5 / (B1 + eps));
+    k[2] = T(1) + (tau5 / (B2 + eps));
+    return;
+  }
+  T epsp = T(1e-6);
+  if (is_mode == IS_SZ10) {
+    epsp = T(1e-10);
+    const T minB = min3(B0, B1, B2), maxB = max3(B0, B1, B2);
+    const T R0 = minB / (maxB + epsp);
+    B0 = R0 * sz10A * minB + B0;
+    B1 = R0 * sz10A * minB + B1;
+    B2 = R0 * sz10A * minB + B2;
+  }
+  k[0] = (epsp + B0) * (epsp + B0);
+  k[1] = (epsp + B1) * (epsp + B1);
+  k[2] = (epsp + B2) * (epsp + B2);
+}
+
+// The face value on one side from the indicators: centre-to-right (c2r = true) or
+// centre-to-left.
+template <class T>
+__device__ __forceinline__ T weno5_side(int is_mode, const T *k, T vm2, T vm1, T v0, T vp1, T vp2, bool c2r)
 {
   // coefficient tables CeesC2R_FV / CeesC2L_FV and DeesC2R_FV / DeesC2L_FV (weno.c:21-28)
   T c00, c01, c02, c10, c11, c12, c20, c21, c22, d0, d1, d2;
@@ -641,37 +781,103 @@ __device__ __forceinline__ T weno5(int is_mode, T sz10A, T vm2, T vm1, T v0, T v
   const T vs0 = c00 * v0 + c01 * vp1 + c02 * vp2;
   const T vs1 = c10 * vm1 + c11 * v0 + c12 * vp1;
   const T vs2 = c20 * vm2 + c21 * vm1 + c22 * v0;
-  const T t0a = T(1) * v0 - T(2) * vp1 + T(1) * vp2, t0b = T(3) * v0 - T(4) * vp1 + T(1) * vp2;
-  const T t1a = T(1) * vm1 - T(2) * v0 + T(1) * vp1, t1b = T(1) * vm1 - T(0) * v0 - T(1) * vp1;
-  const T t2a = T(1) * vm2 - T(2) * vm1 + T(1) * v0, t2b = T(1) * vm2 - T(4) * vm1 + T(3) * v0;
-  T B0 = T(13. / 12.) * (t0a * t0a) + T(1. / 4.) * (t0b * t0b);
-  T B1 = T(13. / 12.) * (t1a * t1a) + T(1. / 4.) * (t1b * t1b);
-  T B2 = T(13. / 12.) * (t2a * t2a) + T(1. / 4.) * (t2b * t2b);
   T w0, w1, w2;
   if (is_mode == IS_B08) {
-    const T eps = T(1e-14);
-    const T tau5 = m_abs(B0 - B2);
-    w0 = d0 * (T(1) + (tau5 / (B0 + eps)));
-    w1 = d1 * (T(1) + (tau5 / (B1 + eps)));
-    w2 = d2 * (T(1) + (tau5 / (B2 + eps)));
-  } else if (is_mode == IS_SZ10) {
-    const T epsp = T(1e-10);
-    const T minB = min3(B0, B1, B2), maxB = max3(B0, B1, B2);
-    const T R0 = minB / (maxB + epsp);
-    B0 = R0 * sz10A * minB + B0;
-    B1 = R0 * sz10A * minB + B1;
-    B2 = R0 * sz10A * minB + B2;
-    w0 = d0 / ((epsp + B0) * (epsp + B0));
-    w1 = d1 / ((epsp + B1) * (epsp + B1));
-    w2 = d2 / ((epsp + B2) * (epsp + B2));
+    w0 = d0 * k[0];
+    w1 = d1 * k[1];
+    w2 = d2 * k[2];
   } else {
-    const T epsp = T(1e-6);
-    w0 = d0 / ((epsp + B0) * (epsp + B0));
-    w1 = d1 / ((epsp + B1) * (epsp + B1));
-    w2 = d2 / ((epsp + B2) * (epsp + B2));
+    w0 = d0 / k[0];
+    w1 = d1 / k[1];
+    w2 = d2 / k[2];
   }
   const T wtot = w0 + w1 + w2;
   return (w0 * vs0 + w1 * vs1 + w2 * vs2) / wtot;
+}
+
+// FP32 WENO5 of one zone, the same scheme from the four first differences D0..D3 of the stencil:
+// the face values as v0 plus a weighted correction (each candidate two operations instead of
+// three, and the correction's rounding instead of the value's), and the JS96 / SZ10 weights
+// from the reciprocals of eps + B (three per zone instead of three per face).
+struct Weno32 {
+  float D0, D1, D2, D3, k0, k1, k2;
+};
+__device__ __forceinline__ Weno32 weno32(int is_mode, float sz10A, float vm2, float vm1, float v0, float vp1, float vp2)
+{
+  Weno32 w;
+  w.D0 = vm1 - vm2;
+  w.D1 = v0 - vm1;
+  w.D2 = vp1 - v0;
+  w.D3 = vp2 - vp1;
+  const float a0 = w.D3 - w.D2, b0 = 3.f * w.D2 - w.D3, a1 = w.D2 - w.D1, b1 = w.D1 + w.D2, a2 = w.D1 - w.D0,
+              b2 = 3.f * w.D1 - w.D0;
+  float B0 = (13.f / 12.f) * (a0 * a0) + 0.25f * (b0 * b0);
+  float B1 = (13.f / 12.f) * (a1 * a1) + 0.25f * (b1 * b1);
+  float B2 = (13.f / 12.f) * (a2 * a2) + 0.25f * (b2 * b2);
+  if (is_mode == IS_B08) {
+    const float tau5 = fabsf(B0 - B2);
+    w.k0 = 1.f + tau5 / (B0 + 1e-14f);
+    w.k1 = 1.f + tau5 / (B1 + 1e-14f);
+    w.k2 = 1.f + tau5 / (B2 + 1e-14f);
+    return w;
+  }
+  float epsp = 1e-6f;
+  if (is_mode == IS_SZ10) {
+    epsp = 1e-10f;
+    const float minB = min3(B0, B1, B2), maxB = max3(B0, B1, B2);
+    const float c = minB / (maxB + epsp) * sz10A * minB;
+    B0 += c;
+    B1 += c;
+    B2 += c;
+  }
+  const float i0 = 1.f / (epsp + B0), i1 = 1.f / (epsp + B1), i2 = 1.f / (epsp + B2);
+  w.k0 = i0 * i0;
+  w.k1 = i1 * i1;
+  w.k2 = i2 * i2;
+  return w;
+}
+__device__ __forceinline__ float weno32_hi(const Weno32 &w, float v0)
+{
+  const float e0 = 0.625f * w.D2 - 0.125f * w.D3, e1 = 0.125f * w.D1 + 0.375f * w.D2, e2 = 0.875f * w.D1 - 0.375f * w.D0;
+  const float w0 = 0.3125f * w.k0, w1 = 0.625f * w.k1, w2 = 0.0625f * w.k2;
+  return v0 + (w0 * e0 + w1 * e1 + w2 * e2) / (w0 + w1 + w2);
+}
+__device__ __forceinline__ float weno32_lo(const Weno32 &w, float v0)
+{
+  const float e0 = 0.375f * w.D3 - 0.875f * w.D2, e1 = -0.375f * w.D1 - 0.125f * w.D2, e2 = 0.125f * w.D0 - 0.625f * w.D1;
+  const float w0 = 0.0625f * w.k0, w1 = 0.625f * w.k1, w2 = 0.3125f * w.k2;
+  return v0 + (w0 * e0 + w1 * e1 + w2 * e2) / (w0 + w1 + w2);
+}
+
+// WENO5 finite-volume, centre-to-right (c2r = true) or centre-to-left face, on the stencil
+// v[-2..2] given as (vm2, vm1, v0, vp1, vp2).
+template <class T>
+__device__ __forceinline__ T weno5(int is_mode, T sz10A, T vm2, T vm1, T v0, T vp1, T vp2, bool c2r)
+{
+  if constexpr (sizeof(T) < sizeof(double)) {
+    const Weno32 w = weno32(is_mode, sz10A, vm2, vm1, v0, vp1, vp2);
+    return c2r ? weno32_hi(w, v0) : weno32_lo(w, v0);
+  } else {
+    T k[3];
+    weno5_indicators(is_mode, sz10A, vm2, vm1, v0, vp1, vp2, k);
+    return weno5_side(is_mode, k, vm2, vm1, v0, vp1, vp2, c2r);
+  }
+}
+
+// Both face values of the zone v0 (lo toward vm1, hi toward vp1) from one set of indicators.
+template <class T>
+__device__ __forceinline__ void weno5_zone(int is_mode, T sz10A, T vm2, T vm1, T v0, T vp1, T vp2, T &lo, T &hi)
+{
+  if constexpr (sizeof(T) < sizeof(double)) {
+    const Weno32 w = weno32(is_mode, sz10A, vm2, vm1, v0, vp1, vp2);
+    lo = weno32_lo(w, v0);
+    hi = weno32_hi(w, v0);
+  } else {
+    T k[3];
+    weno5_indicators(is_mode, sz10A, vm2, vm1, v0, vp1, vp2, k);
+    lo = weno5_side(is_mode, k, vm2, vm1, v0, vp1, vp2, false);
+    hi = weno5_side(is_mode, k, vm2, vm1, v0, vp1, vp2, true);
+  }
 }
 
 // ---- Riemann solvers ------------------------------------------------------------------------
@@ -977,50 +1183,6 @@ __device__ __forceinline__ int hlld_newton(const HlldEqn<T> &q, T &x)
   return 0;
 }
 
-// Secant iteration on equation 48 (the structure of SecantMethodSolver::Solve,
-// Mara/secant.cpp:19-60, which the reference constructs for this equation but does not
-// call): one evaluation per iteration instead of Newton's three.  Used by the FP32-bulk
-// path only; the FP64 path keeps the reference's Newton-Raphson.
-template <class T>
-__device__ __forceinline__ int hlld_secant(const HlldEqn<T> &q, T &x)
-{
-  using Tol = RmhdTol<T>;
-  const int MaxIterations = 15;
-  T x0 = x, x1 = x + T(Tol::jac_dp), y0 = T(0), y1 = T(0);
-  int worse = 0;
-#pragma unroll 1
-  for (int it = -2; it <= MaxIterations; ++it) {
-    // it == -2, -1: the two starting points; then one secant step per iteration
-    T xe;
-    if (it == -2) xe = x0;
-    else if (it == -1) xe = x1;
-    else xe = x1 - y1 * (x1 - x0) / (y1 - y0);
-    T r;
-    if (hlld_function(q, xe, r)) return 1;
-    if (isnan(r)) return 1;
-    if (it == -2) {
-      y0 = r;
-      if (m_abs(y0) < T(Tol::newton_eps)) return 0;
-      continue;
-    }
-    if (it >= 0) {
-      x0 = x1;
-      y0 = y1;
-      x1 = xe;
-    }
-    y1 = r;
-    if (it >= 0) {
-      worse += (m_abs(y1) > m_abs(y0));
-      if (worse >= 10) return 1;
-    }
-    if (m_abs(y1) <= T(Tol::newton_eps)) {
-      x = x1;
-      return 0;
-    }
-  }
-  return 1;
-}
-
 // ReconstructSolution (riemann_hlld-rmhd.cpp:453-575) at s = 0, flux only.
 template <class T>
 __device__ __forceinline__ int hlld_reconstruct(const HlldEqn<T> &q, T p, T *F)
@@ -1068,22 +1230,9 @@ __device__ __forceinline__ int hlld_reconstruct(const HlldEqn<T> &q, T p, T *F)
   const HlldInner<T> &a = left ? aL : aR;
   const T *Uo = left ? q.Ul : q.Ur;
   const T wave = left ? am : ap;
-  // The outer flux.  FP32 bulk recovers it from the jump across the fast wave, Fo = wave Uo - J,
-  // so that Fl and Fr are dead through the pressure iteration (sixteen registers); FP64 keeps
-  // the stored flux.
   T Fo[8];
-  if constexpr (sizeof(T) < sizeof(double)) {
-    Fo[ddd] = wave * Uo[ddd] - J.D;
-    Fo[tau] = wave * Uo[tau] - J.E;
 #pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      Fo[Sx + k] = wave * Uo[Sx + k] - J.m[k];
-      Fo[Bx + k] = wave * Uo[Bx + k] - J.B[k];
-    }
-  } else {
-#pragma unroll
-    for (int i = 0; i < 8; ++i) Fo[i] = left ? q.Fl[i] : q.Fr[i];
-  }
+  for (int i = 0; i < 8; ++i) Fo[i] = left ? q.Fl[i] : q.Fr[i];
   if (region == 0 || region == 5) {
 #pragma unroll
     for (int i = 0; i < 8; ++i) F[i] = Fo[i];
@@ -1137,110 +1286,6 @@ __device__ __forceinline__ int hlld_reconstruct(const HlldEqn<T> &q, T p, T *F)
   return 0;
 }
 
-// First attempt of the HLL-state c2p in the FP32-bulk HLLD: the Anton et al. 2-D Newton of
-// c2p_anton2dzw_fast in FP32 from the average face state (in P), to a step tolerance of 1e-6,
-// with the reference's clamps, reconstruction, pressure floor and checks.  The HLL state's
-// primitives only seed the eq. 48 pressure guess and are kept in FP32 anyway, so an FP32
-// polish loses nothing; returns nonzero (the caller then runs the FP64 ladder) when the state
-// fails check_cons, the guess is unusable, Newton does not converge in 32 iterations or the
-// primitives fail check_prim.
-__device__ __forceinline__ int c2p_hll_f32(const PhysParams &pp, const float *U, float *P, int &iters)
-{
-  iters = 0;
-  if (check_cons(U)) return 1;
-  const float V2g = P[vx] * P[vx] + P[vy] * P[vy] + P[vz] * P[vz];
-  if (!(V2g < 1.f && P[rho] > 0.f && P[pre] > 0.f)) return 1;
-  const float gamma = float(pp.gamma), gamf = (gamma - 1.f) / gamma;
-  const float D = U[ddd], Tau = U[tau];
-  const float S2 = U[Sx] * U[Sx] + U[Sy] * U[Sy] + U[Sz] * U[Sz];
-  const float B2 = U[Bx] * U[Bx] + U[By] * U[By] + U[Bz] * U[Bz];
-  const float BS = U[Bx] * U[Sx] + U[By] * U[Sy] + U[Bz] * U[Sz];
-  const float BS2 = BS * BS;
-  const float W2g = 1.f / (1.f - V2g);
-  float Z = P[rho] * (1.f + P[pre] / P[rho] * (1.f / (gamma - 1.f) + 1.f)) * W2g;
-  float W = sqrtf(W2g);
-  const float iD = 1.f / D;
-  float iW = 1.f / W, iZ = 1.f / Z;
-  float error = 1.f;
-  while (error > 1e-6f) {
-    const float W2 = W * W, Z2 = Z * Z, Z3 = Z * Z2;
-    const float iW2 = iW * iW, iW3 = iW2 * iW, iZ2 = iZ * iZ, iZ3 = iZ2 * iZ;
-    const float Pre = D * iW * (Z * iD * iW - 1.f) * gamf;
-    const float BZ = B2 + Z;
-    const float df0dZ = 2.f * BZ * (BS2 * W2 + (W2 - 1.f) * Z3) * iW2 * iZ3;
-    const float df0dW = 2.f * BZ * BZ * iW3;
-    const float df1dZ = 1.f + BS2 * iZ3 - gamf * iW2;
-    const float df1dW = (B2 + (2.f * Z - D * W) * gamf) * iW3;
-    const float f0 = -S2 + BZ * BZ * (W2 - 1.f) * iW2 - (2.f * Z + B2) * BS2 * iZ2;
-    const float f1 = -Tau + Z + B2 - Pre - 0.5f * B2 * iW2 - 0.5f * BS2 * iZ2 - D;
-    const float idet = 1.f / (df0dZ * df1dW - df0dW * df1dZ);
-    const float dZ = -(df1dW * f0 - df0dW * f1) * idet;
-    const float dW = -(df0dZ * f1 - df1dZ * f0) * idet;
-    float Zn = fabsf(Z + dZ), Wn = W + dW;
-    Zn = (Zn < 1e20f) ? Zn : Z;
-    Wn = fminf(fmaxf(Wn, 1.f), 1e12f);
-    Z = Zn;
-    W = Wn;
-    iZ = 1.f / Z;
-    iW = 1.f / W;
-    error = fabsf(dZ * iZ) + fabsf(dW * iW);
-    if (!(error == error) || ++iters == 32) return 1;
-  }
-  float Q[8];
-  const float b0 = BS * W * iZ;
-  Q[rho] = D * iW;
-  Q[pre] = D * iW * (Z * iD * iW - 1.f) * gamf;
-  const float iZB = 1.f / (Z + B2);
-  Q[vx] = (U[Sx] + b0 * U[Bx] * iW) * iZB;
-  Q[vy] = (U[Sy] + b0 * U[By] * iW) * iZB;
-  Q[vz] = (U[Sz] + b0 * U[Bz] * iW) * iZB;
-  Q[Bx] = U[Bx];
-  Q[By] = U[By];
-  Q[Bz] = U[Bz];
-  if (pp.pfloor > 0.0 && Q[pre] < float(pp.pfloor)) Q[pre] = float(pp.pfloor);
-  if (check_prim(Q)) return 1;
-#pragma unroll
-  for (int i = 0; i < 8; ++i) P[i] = Q[i];
-  return 0;
-}
-
-// Converts a flux-solver state to double for the FP64 c2p and back.  P holds the average of
-// the two face states on entry.  The FP64 path runs the reference's ladder as it is (first
-// attempt from the estimate of the conserved state).  The FP32-bulk path first tries
-// c2p_hll_f32; when that fails it runs the FP64 Newton from the average state -- in smooth
-// flow the HLL state's primitives are close to it, so that polish takes 2 iterations instead
-// of 6 (measured, 256^3 turbulence) -- and then the estimate and the reference ladder; the
-// root it lands on is the same to the Newton tolerance.
-template <class T>
-__device__ __forceinline__ int cons_to_prim_T(const PhysParams &pp, const T *U, T *P, C2PTally *tally)
-{
-  if constexpr (sizeof(T) < sizeof(double)) {
-    int it = 0;
-    if (c2p_hll_f32(pp, U, P, it) == 0) {
-      if (tally) { tally->iters = it; tally->attempts = 1; }
-      return 0;
-    }
-  }
-  double Ud[8], Pd[8];
-#pragma unroll
-  for (int i = 0; i < 8; ++i) { Ud[i] = double(U[i]); Pd[i] = double(P[i]); }
-  int e;
-  if constexpr (sizeof(T) < sizeof(double)) {
-    const double V2 = Pd[vx] * Pd[vx] + Pd[vy] * Pd[vy] + Pd[vz] * Pd[vz];
-    const double W2 = 1.0 / (1.0 - V2);
-    const double h = 1.0 + Pd[pre] / Pd[rho] * (1.0 / (pp.gamma - 1.0) + 1.0);   // 1 + e + p/rho
-    const bool usable = V2 < 1.0 && Pd[rho] > 0.0 && Pd[pre] > 0.0;
-    e = cons_to_prim<true, 1>(pp, Ud, Pd, tally, Pd[rho] * h * W2, sqrt(W2), usable);
-  } else {
-    e = cons_to_prim<false, 2>(pp, Ud, Pd, tally);
-  }
-  if (e == 0) {
-#pragma unroll
-    for (int i = 0; i < 8; ++i) P[i] = T(Pd[i]);
-  }
-  return e;
-}
-
 // HLL total pressure, EstimateSolution(0) (riemann_hlld-rmhd.cpp:543-553), from the HLL
 // state's primitives.
 template <class T>
@@ -1273,28 +1318,17 @@ __device__ __forceinline__ T hlld_estimate1(T E, T FE, T m, T Fm)
 // HlldRmhdRiemannSolver::IntercellFlux at s = 0 (riemann_hlld-rmhd.cpp:179-313).
 // Returns 1 when a face state is unphysical (the caller retries with PCM states);
 // `used_hllc` reports the fallback.
-// A thread's slot for the HLLD equation state in shared memory (53 words: an odd stride, so
-// the threads of a warp hit different banks).
-template <class T>
-struct HlldSlot {
-  HlldEqn<T> q;
-  T pad;
-};
-
-// slot: where the equation state lives through the pressure iteration -- nullptr for
-// registers (the compiler's choice), or this thread's HlldSlot in shared memory, so that the
-// ~50 values are read from there when needed instead of occupying registers throughout.
 template <class T, int dim>
 __device__ __forceinline__ int riemann_hlld(const PhysParams &pp, const T *pl, const T *pr, T *f, T &ml,
-                                         int &used_hllc, C2PTally *tally, HlldSlot<T> *slot = nullptr)
+                                         int &used_hllc, C2PTally *tally)
 {
+  static_assert(sizeof(T) == sizeof(double), "FP32 faces take riemann_hlld32 (rmhd_face32.cuh)");
   using Tol = RmhdTol<T>;
   const T gamma = T(pp.gamma);
   using M = DimMap<dim>;
   constexpr int B1 = M::B1, B2 = M::B2, B3 = M::B3, S1 = M::S1, S2 = M::S2, S3 = M::S3;
   constexpr int v1 = M::v1, v2 = M::v2, v3 = M::v3;
-  HlldEqn<T> q_regs;
-  HlldEqn<T> &q = slot ? slot->q : q_regs;
+  HlldEqn<T> q;
   T Pl[8], Pr[8], epl, eml, epr, emr;
   Pl[pre] = pl[pre]; Pr[pre] = pr[pre];
   Pl[rho] = pl[rho]; Pr[rho] = pr[rho];
@@ -1321,15 +1355,7 @@ __device__ __forceinline__ int riemann_hlld(const PhysParams &pp, const T *pl, c
     U_hll[i] = (ap * q.Ur[i] - am * q.Ul[i] + (q.Fl[i] - q.Fr[i])) / (ap - am);
     F_hll[i] = (ap * q.Fl[i] - am * q.Fr[i] + ap * am * (q.Ur[i] - q.Ul[i])) / (ap - am);
   }
-  const int hll_c2p_failed = cons_to_prim_T(pp, U_hll, P_hll, tally);
-  // FP32 bulk takes both pressure estimates here, so that P_hll, U_hll and F_hll are dead
-  // through the pressure iteration; FP64 keeps the reference's order (and its in-place shift
-  // and restore of tau, which the Bx ~ 0 retries repeat).
-  T p_est0 = T(0), p_est1 = T(0);
-  if constexpr (sizeof(T) < sizeof(double)) {
-    p_est0 = hlld_estimate0(P_hll);
-    p_est1 = hlld_estimate1(U_hll[tau] + U_hll[ddd], F_hll[tau] + F_hll[ddd], U_hll[Sx], F_hll[Sx]);
-  }
+  const int hll_c2p_failed = cons_to_prim<false, 2>(pp, U_hll, P_hll, tally);
   // HlldEquation48 constructor (riemann_hlld-rmhd.cpp:315-345)
   q.ap = ap; q.am = am; q.PlBx = Pl[Bx]; q.PrBx = Pr[Bx];
   q.Ul[tau] += q.Ul[ddd];
@@ -1353,9 +1379,7 @@ __device__ __forceinline__ int riemann_hlld(const PhysParams &pp, const T *pl, c
     T p_star;
     int rc;
     const int est = (m_abs(Pl[Bx]) < T(Tol::bx_small) || m_abs(Pr[Bx]) < T(Tol::bx_small)) ? 1 : attempt;
-    if constexpr (sizeof(T) < sizeof(double)) {
-      p_star = est == 0 ? p_est0 : (est == 1 ? p_est1 : T(0));
-    } else if (est == 0) {
+    if (est == 0) {
       p_star = hlld_estimate0(P_hll);
     } else if (est == 1) {   // EstimateSolution(1) shifts tau and restores it afterwards
       F_hll[tau] += F_hll[ddd];
@@ -1369,7 +1393,7 @@ __device__ __forceinline__ int riemann_hlld(const PhysParams &pp, const T *pl, c
     if (m_abs(Pl[Bx]) < T(Tol::bx_small) || m_abs(Pr[Bx]) < T(Tol::bx_small)) {
       rc = hlld_reconstruct(q, p_star, F);
     } else {
-      rc = sizeof(T) < sizeof(double) ? hlld_secant(q, p_star) : hlld_newton(q, p_star);
+      rc = hlld_newton(q, p_star);
       if (rc == 0) rc = hlld_reconstruct(q, p_star, F);
     }
     success = (rc == 0);

@@ -12,12 +12,16 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
-#include "rmhd_physics.cuh"
+#include "rmhd_face32.cuh"
 
 // Minimum resident blocks of 128 threads per SM requested for the flux sweep (caps its
 // registers at 65536 / (128 * MGPU_FLUX_MINB)).
 #ifndef MGPU_FLUX_MINB
 #define MGPU_FLUX_MINB 2
+#endif
+// The same for the HLLD sweeps.
+#ifndef MGPU_HLLD_MINB
+#define MGPU_HLLD_MINB MGPU_FLUX_MINB
 #endif
 // The same for the zone c2p kernel (5 blocks: chosen by a sweep of 3-5; its natural register
 // count allows 3).
@@ -91,6 +95,12 @@ __device__ __forceinline__ void warp_add(unsigned long long *ctr, unsigned v)
   const unsigned mask = __activemask();
   const unsigned sum = __reduce_add_sync(mask, v);
   if ((threadIdx.x & 31) == __ffs(mask) - 1 && sum) atomicAdd(ctr, (unsigned long long) sum);
+}
+
+// Minimum resident blocks of the sweeps of Riemann solver RS.
+template <int RS> __host__ __device__ constexpr int flux_minb()
+{
+  return RS == RIEMANN_HLLD ? MGPU_HLLD_MINB : MGPU_FLUX_MINB;
 }
 
 // ---- begin: dt and counters ----------------------------------------------------------------
@@ -329,31 +339,78 @@ struct FluxTally {
   int hlld_ok, hlld_hllc, pcm_retry, face_c2p_calls, face_c2p_iters;
 };
 
-// One face: reconstruct, Riemann solve (PCM retry on failure), the flux in Fo (zero when both
-// attempts fail); the face's |lambda| is folded into ml.
-template <class T, int dim, int RS>
-__device__ __forceinline__ void face_flux(const Grid &g, const T *__restrict__ PA, const PhysParams &pp, long long f,
-                                          T &ml, FluxTally &ft, T *Fo, HlldSlot<T> *slot = nullptr)
+// The two states of the face between zones f and f + S: reconstructed, or with retry the zone
+// states themselves.  The reconstruction is chosen once, outside the component loops, so that
+// each loop's loads are issued together.
+template <class T>
+__device__ __forceinline__ void face_states(const T *__restrict__ PA, long long cs, long long S, const PhysParams &pp,
+                                            long long f, bool retry, T *Pl, T *Pr)
 {
-  const long long S = g.s[dim - 1];
-  T Pl[8], Pr[8];
-  const T theta = T(pp.theta);
+  const T *a = PA + f;
+  if (retry || pp.recon == RECON_PCM) {
 #pragma unroll
-  for (int q = 0; q < 8; ++q) {
-    const T *a = PA + q * g.cs + f;
-    if (pp.recon == RECON_PCM) {
+    for (int q = 0; q < 8; ++q, a += cs) {
       Pl[q] = a[0];
       Pr[q] = a[S];
-    } else if (pp.recon == RECON_PLM) {
+    }
+  } else if (pp.recon == RECON_PLM) {
+    const T theta = T(pp.theta);
+#pragma unroll
+    for (int q = 0; q < 8; ++q, a += cs) {
       const T vm = a[-S], v0 = a[0], vp = a[S], vpp = a[2 * S];
       Pl[q] = plm(theta, vm, v0, vp, T(+1));
       Pr[q] = plm(theta, v0, vp, vpp, T(-1));
-    } else {
+    }
+  } else {
+#pragma unroll
+    for (int q = 0; q < 8; ++q, a += cs) {
       const T vm2 = a[-2 * S], vm1 = a[-S], v0 = a[0], vp1 = a[S], vp2 = a[2 * S], vp3 = a[3 * S];
       Pl[q] = weno5(pp.is_mode, T(pp.sz10A), vm2, vm1, v0, vp1, vp2, true);
       Pr[q] = weno5(pp.is_mode, T(pp.sz10A), vm1, v0, vp1, vp2, vp3, false);
     }
   }
+}
+
+// Both face values of zone z along stride S: lo toward z - S, hi toward z + S, which are
+// face_states' Pr of the face below and Pl of the face above.
+template <class T>
+__device__ __forceinline__ void zone_states(const T *__restrict__ PA, long long cs, long long S, const PhysParams &pp,
+                                            long long z, T *lo, T *hi)
+{
+  const T *a = PA + z;
+  if (pp.recon == RECON_PCM) {
+#pragma unroll
+    for (int q = 0; q < 8; ++q, a += cs) lo[q] = hi[q] = a[0];
+  } else if (pp.recon == RECON_PLM) {
+    const T theta = T(pp.theta);
+#pragma unroll
+    for (int q = 0; q < 8; ++q, a += cs) plm_zone(theta, a[-S], a[0], a[S], lo[q], hi[q]);
+  } else {
+#pragma unroll
+    for (int q = 0; q < 8; ++q, a += cs)
+      weno5_zone(pp.is_mode, T(pp.sz10A), a[-2 * S], a[-S], a[0], a[S], a[2 * S], lo[q], hi[q]);
+  }
+}
+
+// A face's states fetched again on the rare paths of the FP32 HLLD solver (out of line).
+struct FaceStates32 {
+  float l[8], r[8];
+};
+static __device__ __noinline__ FaceStates32 refetch_face(const float *PA, long long cs, long long S, PhysParams pp,
+                                                         long long f, bool retry)
+{
+  FaceStates32 o;
+  face_states<float>(PA, cs, S, pp, f, retry, o.l, o.r);
+  return o;
+}
+
+// The flux of the face between zones f and f + S from its states Pl, Pr (overwritten by the PCM
+// retry), in Fo (zero when both attempts fail); the face's |lambda| is folded into ml.
+template <class T, int dim, int RS>
+__device__ __forceinline__ void solve_face(const Grid &g, const T *__restrict__ PA, const PhysParams &pp, long long f,
+                                           T *Pl, T *Pr, T &ml, FluxTally &ft, T *Fo)
+{
+  const long long S = g.s[dim - 1];
   const T gamma = T(pp.gamma);
   int err = 1, used_hllc = 0;
   constexpr bool hlld = RS == RIEMANN_HLLD;
@@ -371,7 +428,17 @@ __device__ __forceinline__ void face_flux(const Grid &g, const T *__restrict__ P
       }
     }
     C2PTally t{0, 0};
-    if constexpr (RS == RIEMANN_HLLD) err = riemann_hlld<T, dim>(pp, Pl, Pr, Fo, ml, used_hllc, &t, slot);
+    if constexpr (RS == RIEMANN_HLLD && sizeof(T) < sizeof(double)) {
+      const auto src = [&](float *l, float *r) {
+        const FaceStates32 o = refetch_face(PA, g.cs, S, pp, f, attempt == 1);
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          l[q] = o.l[q];
+          r[q] = o.r[q];
+        }
+      };
+      err = riemann_hlld32<dim>(pp, Pl, Pr, Fo, ml, used_hllc, &t, src);
+    } else if constexpr (RS == RIEMANN_HLLD) err = riemann_hlld<T, dim>(pp, Pl, Pr, Fo, ml, used_hllc, &t);
     else if constexpr (RS == RIEMANN_HLLC) err = riemann_hllc<T, dim>(gamma, Pl, Pr, Fo, ml);
     else err = riemann_hll<T, dim>(gamma, Pl, Pr, Fo, ml);
     tally.iters += t.iters;
@@ -387,6 +454,16 @@ __device__ __forceinline__ void face_flux(const Grid &g, const T *__restrict__ P
   }
   ft.face_c2p_calls += tally.attempts > 0;
   ft.face_c2p_iters += tally.iters;
+}
+
+// One face: reconstruct and solve.
+template <class T, int dim, int RS>
+__device__ __forceinline__ void face_flux(const Grid &g, const T *__restrict__ PA, const PhysParams &pp, long long f,
+                                          T &ml, FluxTally &ft, T *Fo)
+{
+  T Pl[8], Pr[8];
+  face_states<T>(PA, g.cs, g.s[dim - 1], pp, f, false, Pl, Pr);
+  solve_face<T, dim, RS>(g, PA, pp, f, Pl, Pr, ml, ft, Fo);
 }
 
 // One face, its flux stored in F.
@@ -428,7 +505,7 @@ __device__ __forceinline__ void flux_block_finish(double m, const FluxTally &ft,
 }
 
 template <class T, int dim, int RS>
-__global__ void __launch_bounds__(128, MGPU_FLUX_MINB) k_flux(Grid g, const T *__restrict__ PA, T *__restrict__ F,
+__global__ void __launch_bounds__(128, flux_minb<RS>()) k_flux(Grid g, const T *__restrict__ PA, T *__restrict__ F,
                                                               PhysParams pp, Ctl *ctl, int stage)
 {
   if (stage_failed(ctl, stage + 1)) return;
