@@ -2,7 +2,7 @@
 #ifdef MGPU_FLUX_MINB_OVERRIDE
 #define MGPU_FLUX_MINB MGPU_FLUX_MINB_OVERRIDE
 #else
-#define MGPU_FLUX_MINB 4
+#define MGPU_FLUX_MINB 5
 #endif
 // HLLD sweeps (rmhd_face32.cuh) at 6 blocks, 80 registers: 160^3 lean sweeps per RK3 step 3.82 /
 // 3.34 / 3.29 ms (PLM) and 5.80 / 4.86 / 4.75 ms (WENO5) at 4 / 5 / 6 blocks

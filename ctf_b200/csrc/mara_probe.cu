@@ -98,7 +98,20 @@ __device__ int riemann_dim(int solver, const PhysParams &pp, const double *pl, c
   if (solver == RIEMANN_HLL) return riemann_hll<double, dim>(pp.gamma, pl, pr, f, ml);
   if (solver == RIEMANN_HLLC) return riemann_hllc<double, dim>(pp.gamma, pl, pr, f, ml);
   C2PTally t{0, 0};
-  return riemann_hlld<double, dim>(pp, pl, pr, f, ml, used_hllc, &t);
+  const auto src = [&](double *l, double *r) {
+    for (int q = 0; q < 8; ++q) {
+      l[q] = pl[q];
+      r[q] = pr[q];
+    }
+  };
+  double states[32], F[8];
+  for (int q = 0; q < 8; ++q) {
+    states[q] = pl[frame_slot(dim, q)];
+    states[8 + q] = pr[frame_slot(dim, q)];
+  }
+  const int err = riemann_hlld64(pp, dim, Column<double>{states, 1}, F, ml, used_hllc, &t, src);
+  for (int q = 0; q < 8; ++q) f[frame_slot(dim, q)] = F[q];
+  return err;
 }
 
 // dims: per-face direction (1-3) when not null, else `dim` for every face.

@@ -62,35 +62,35 @@ __device__ __forceinline__ void warp_add_int(int *ctr, int v)
   if ((threadIdx.x & 31) == __ffs(mask) - 1 && sum) atomicAdd(ctr, sum);
 }
 
-// RiemannSolver::IntercellFlux at s = 0 of the compile-time solver; 0 on success.
+// RiemannSolver::IntercellFlux at s = 0 of the compile-time solver; 0 on success.  States and flux
+// in face_slot's order.
 template <class T, int dim, int RS>
 __device__ __forceinline__ int ctu_riemann(const PhysParams &pp, const T *Pl, const T *Pr, T *Fo, T &ml,
-                                           FluxTally &ft)
+                                           FluxTally &ft, T *colp)
 {
-  int err;
-  if constexpr (RS == RIEMANN_HLLD) {
-    C2PTally t{0, 0};
-    int used_hllc = 0;
-    if constexpr (sizeof(T) < sizeof(double)) {
-      const auto src = [&](float *l, float *r) {
+  C2PTally t{0, 0};
+  int used_hllc = 0;
+  const Column<T> col{colp, 128};
+  if constexpr (uses_column<T, RS>()) {
 #pragma unroll
-        for (int q = 0; q < 8; ++q) {
-          l[q] = Pl[q];
-          r[q] = Pr[q];
-        }
-      };
-      err = riemann_hlld32<dim>(pp, Pl, Pr, Fo, ml, used_hllc, &t, src);
-    } else {
-      err = riemann_hlld<T, dim>(pp, Pl, Pr, Fo, ml, used_hllc, &t);
+    for (int q = 0; q < 8; ++q) {
+      col[q] = Pl[q];
+      col[8 + q] = Pr[q];
     }
+  }
+  const auto src = [&](T *l, T *r) {
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      l[face_slot<T, RS>(dim, q)] = Pl[q];
+      r[face_slot<T, RS>(dim, q)] = Pr[q];
+    }
+  };
+  const int err = riemann_face<T, RS>(pp, dim, Pl, Pr, Fo, ml, used_hllc, &t, col, src);
+  if constexpr (RS == RIEMANN_HLLD) {
     ft.hlld_ok += 1 - used_hllc;
     ft.hlld_hllc += used_hllc;
     ft.face_c2p_calls += t.attempts > 0;
     ft.face_c2p_iters += t.iters;
-  } else if constexpr (RS == RIEMANN_HLLC) {
-    err = riemann_hllc<T, dim>(T(pp.gamma), Pl, Pr, Fo, ml);
-  } else {
-    err = riemann_hll<T, dim>(T(pp.gamma), Pl, Pr, Fo, ml);
   }
   return err;
 }
@@ -111,20 +111,27 @@ __global__ void __launch_bounds__(128, flux_minb<RS>()) k_ctu_flux(Grid g, const
   T ml = T(0);
   FluxTally ft{0, 0, 0, 0, 0};
   int bad = 0;
+  __shared__ T cols[column_entries<T, RS>() * 128];
   if (f < g.nz - sx) {
     T Pl[8], Pr[8], Fo[8];
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
-      const T *a = PA + q * g.cs;
-      const T *b = src + q * g.cs;
+      const T *a = PA + face_slot<T, RS>(dim, q) * g.cs;
+      const T *b = src + face_slot<T, RS>(dim, q) * g.cs;
       Pr[q] = b[f + S] - T(0.5) * ctu_slope(g, a, f + S, S, theta);
       Pl[q] = b[f] + T(0.5) * ctu_slope(g, a, f, S, theta);
     }
-    bad = check_prim(Pl) || check_prim(Pr);
-    const int err = bad ? 1 : ctu_riemann<T, dim, RS>(pp, Pl, Pr, Fo, ml, ft);
+    T ql[8], qr[8];   // in the reference's component order
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      ql[face_slot<T, RS>(dim, q)] = Pl[q];
+      qr[face_slot<T, RS>(dim, q)] = Pr[q];
+    }
+    bad = check_prim(ql) || check_prim(qr);
+    const int err = bad ? 1 : ctu_riemann<T, dim, RS>(pp, Pl, Pr, Fo, ml, ft, cols + threadIdx.x);
     if (pass == 1 || !err) {
 #pragma unroll
-      for (int q = 0; q < 8; ++q) F[q * g.cs + f] = err ? T(0) : Fo[q];
+      for (int q = 0; q < 8; ++q) F[face_slot<T, RS>(dim, q) * g.cs + f] = err ? T(0) : Fo[q];
     }
   }
   flux_block_finish(double(ml), ft, ctl, RS == RIEMANN_HLLD);

@@ -111,6 +111,7 @@ __global__ void __launch_bounds__(128, flux_minb<RS>()) k_ens_flux(const BoxDev 
                                                                   int stage)
 {
   __shared__ BoxDev d;
+  __shared__ T cols[column_entries<T, RS>() * 128];
   constexpr bool hlld = RS == RIEMANN_HLLD;
   for (long long w = blockIdx.x; w < ntiles; w += gridDim.x) {
     const int2 m = map[w];
@@ -123,7 +124,7 @@ __global__ void __launch_bounds__(128, flux_minb<RS>()) k_ens_flux(const BoxDev 
     FluxTally ft{0, 0, 0, 0, 0};
     for (int s = threadIdx.x; s < tile; s += blockDim.x) {
       const long long f = base + s;
-      if (f < end) flux_face<T, dim, RS>(d.g, (const T *) d.b.PA, (T *) d.b.F[dim - 1], pp, f, ml, ft);
+      if (f < end) flux_face<T, RS>(d.g, (const T *) d.b.PA, (T *) d.b.F[dim - 1], pp, dim, f, ml, ft, cols + threadIdx.x);
     }
     flux_block_finish(double(ml), ft, d.ctl, hlld);
   }

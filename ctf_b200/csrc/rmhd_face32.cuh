@@ -1,4 +1,4 @@
-// The FP32-bulk HLLD face, written for FP32 (the FP64 path keeps the reference's expressions in
+// The FP32-bulk HLLC and HLLD faces, written for FP32 (the FP64 path keeps the reference's expressions in
 // rmhd_physics.cuh).
 //
 // The sweeps are bound by instruction issue and latency, so this file spends as few
@@ -90,13 +90,130 @@ __device__ __forceinline__ int side_state(float gamma, float rh_p, float r, floa
   return 0;
 }
 
-// ---- HLLD ------------------------------------------------------------------------------------------
-// One side of the eq. 48 problem: the outer speed and the jump J = lam U - F across it (the
-// normal field's jump is lam Bx).
+// One side's outer speed and the jump J = lam U - F across it (the normal field's is lam Bx).
 struct HlldSide32 {
   float lam, D, E, m0, m1, m2, B1, B2;
 };
 
+__device__ __forceinline__ HlldSide32 side_jump(const SideState &s, float lam)
+{
+  return {lam, lam * s.D - s.FD, lam * s.E - s.S0, lam * s.S0 - s.FS0, lam * s.S1 - s.FS1, lam * s.S2 - s.FS2,
+          lam * s.B1 - s.FB1, lam * s.B2 - s.FB2};
+}
+
+// Both sides of a face from its states pl, pr in the normal frame, the outer speeds and their
+// fold into ml.  Non-zero when a face state is unphysical.
+__device__ __forceinline__ int face_sides(float gamma, const float *pl, const float *pr, float bx, SideState &s,
+                                          SideState &t, float &ap, float &am, float &ml)
+{
+  const float rh_p = gamma / (gamma - 1.f);
+  FastPair fl, fr;
+  if (side_state(gamma, rh_p, pl[rho], pl[pre], pl[vx], pl[vy], pl[vz], bx, pl[By], pl[Bz], s, fl, nullptr)) return 1;
+  if (side_state(gamma, rh_p, pr[rho], pr[pre], pr[vx], pr[vy], pr[vz], bx, pr[By], pr[Bz], t, fr, &fl)) return 1;
+  ap = fmaxf(fl.hi, fr.hi);
+  am = fminf(fl.lo, fr.lo);
+  if (!(ap <= 1.f && am >= -1.f)) {
+    ap = 1.f;
+    am = -1.f;
+  }
+  ml = fmaxf(ml, fmaxf(fabsf(ap), fabsf(am)));
+  return 0;
+}
+
+// ---- HLLC ------------------------------------------------------------------------------------------
+// HllcRmhdRiemannSolver::IntercellFlux at s = 0 (Mara/riemann_hllc-rmhd.cpp:26-178) from the
+// jumps: U_hll = (J_R - J_L) / (ap - am), and the flux lam U* - J of the side of the contact that holds s = 0 (the other side's star state is not
+// formed).  A contact or star state that FP32 made non-finite takes the HLL flux.  pl, pr and f
+// in the normal frame.
+__device__ __forceinline__ int riemann_hllc32(float gamma, const float *pl, const float *pr, float *f, float &ml)
+{
+  using Tol = RmhdTol<float>;
+  const float bx = 0.5f * (pl[Bx] + pr[Bx]);
+  SideState s, t;
+  float ap, am;
+  if (face_sides(gamma, pl, pr, bx, s, t, ap, am, ml)) return 1;
+  f[Bx] = 0.f;
+  if (am >= 0.f || ap < 0.f) {
+    const bool left = am >= 0.f;
+    f[ddd] = left ? s.FD : t.FD;
+    f[tau] = (left ? s.S0 : t.S0) - f[ddd];
+    f[Sx] = left ? s.FS0 : t.FS0;
+    f[Sy] = left ? s.FS1 : t.FS1;
+    f[Sz] = left ? s.FS2 : t.FS2;
+    f[By] = left ? s.FB1 : t.FB1;
+    f[Bz] = left ? s.FB2 : t.FB2;
+    return 0;
+  }
+  const HlldSide32 L = side_jump(s, am), R = side_jump(t, ap);
+  const float is = 1.f / (ap - am);
+  const float UE = (R.E - L.E) * is, U0 = (R.m0 - L.m0) * is, U1 = (R.B1 - L.B1) * is, U2 = (R.B2 - L.B2) * is;
+  // not from the jumps: their difference would cancel ap am U, and w2, w3 divide F1, F2 by bx
+  const float q = ap * am;
+  const float FE = (ap * s.S0 - am * t.S0 + q * (t.E - s.E)) * is, F0 = (ap * s.FS0 - am * t.FS0 + q * (t.S0 - s.S0)) * is,
+              F1 = (ap * s.FB1 - am * t.FB1 + q * (t.B1 - s.B1)) * is,
+              F2 = (ap * s.FB2 - am * t.FB2 + q * (t.B2 - s.B2)) * is;
+  float w1, w2 = 0.f, w3 = 0.f, vdB = 0.f, g2 = 1.f, b1 = 0.f, ps;
+  const bool field = fabsf(bx) > Tol::hllc_bx;
+  if (field) {
+    const float BdFB = U1 * F1 + U2 * F2;
+    w1 = hllc_contact_speed(FE - BdFB, -F0 - UE + (U1 * U1 + U2 * U2) + (F1 * F1 + F2 * F2), U0 - BdFB);
+    const float ib = 1.f / bx;
+    w2 = (U1 * w1 - F1) * ib;
+    w3 = (U2 * w1 - F2) * ib;
+    b1 = bx;
+    vdB = w1 * b1 + w2 * U1 + w3 * U2;
+    g2 = 1.f - (w1 * w1 + w2 * w2 + w3 * w3);
+    ps = F0 + b1 * b1 * g2 - (FE - b1 * vdB) * w1;
+  } else {
+    w1 = hllc_contact_speed(FE, -F0 - UE, U0);
+    ps = F0 - FE * w1;
+  }
+  const bool left = w1 >= 0.f;
+  const float lam = left ? am : ap;
+  const float JD = left ? L.D : R.D, JE = left ? L.E : R.E, J0 = left ? L.m0 : R.m0, J1 = left ? L.m1 : R.m1,
+              J2 = left ? L.m2 : R.m2, JB1 = left ? L.B1 : R.B1, JB2 = left ? L.B2 : R.B2;
+  const float k = 1.f / (lam - w1);
+  const float D = JD * k, E = (JE + ps * w1 - vdB * b1) * k;
+  const float m0 = (E + ps) * w1 - vdB * b1;
+  const float m1 = (J1 - b1 * (U1 * g2 + vdB * w2)) * k, m2 = (J2 - b1 * (U2 * g2 + vdB * w3)) * k;
+  const float c1 = field ? U1 : JB1 * k, c2 = field ? U2 : JB2 * k;
+  if (isfinite(w1) && isfinite(ps) && isfinite(D) && isfinite(E) && isfinite(m1) && isfinite(m2) && isfinite(m0) &&
+      isfinite(c1) && isfinite(c2)) {
+    f[ddd] = lam * D - JD;
+    f[tau] = (lam * E - JE) - f[ddd];
+    f[Sx] = lam * m0 - J0;
+    f[Sy] = lam * m1 - J1;
+    f[Sz] = lam * m2 - J2;
+    f[By] = lam * c1 - JB1;
+    f[Bz] = lam * c2 - JB2;
+  } else {
+    f[ddd] = (am * R.D - ap * L.D) * is;
+    f[tau] = FE - f[ddd];
+    f[Sx] = F0;
+    f[Sy] = (am * R.m1 - ap * L.m1) * is;
+    f[Sz] = (am * R.m2 - ap * L.m2) * is;
+    f[By] = F1;
+    f[Bz] = F2;
+  }
+  return 0;
+}
+
+// The HLLD solver's fallback, out of line (rare); states in the reference's component order.
+static __device__ __noinline__ HllcOut<float> riemann_hllc32_fallback(int dim, float gamma, Face8<float> pl,
+                                                                      Face8<float> pr, float ml)
+{
+  float l[8], r[8];
+  for (int k = 0; k < 8; ++k) {
+    l[k] = pl.v[frame_slot(dim, k)];
+    r[k] = pr.v[frame_slot(dim, k)];
+  }
+  HllcOut<float> o;
+  o.ml = ml;
+  o.err = riemann_hllc32(gamma, l, r, o.F, o.ml);
+  return o;
+}
+
+// ---- HLLD ------------------------------------------------------------------------------------------
 struct HlldInner32 {
   float v0, v1, v2, b1, b2;   // between the fast and Alfven waves
   float ia, w;                // 1 / (lam - v0), total enthalpy
@@ -223,11 +340,9 @@ __device__ __forceinline__ int hlld_flux32(const HlldSide32 &L, const HlldSide32
   if (!((e.r.w > p) && (e.r.v0 < R.lam + TOL) && (cr0 < e.r.K0 + TOL))) return 1;
   if (fabsf(cr0 - cl0) > Tol::contact) return 1;
   const bool left = lamC >= 0.f;
-  const HlldSide32 &J = left ? L : R;
   const float lam = left ? L.lam : R.lam;
   const float JD = left ? L.D : R.D, JE = left ? L.E : R.E, m0 = left ? L.m0 : R.m0, m1 = left ? L.m1 : R.m1,
               m2 = left ? L.m2 : R.m2, JB1 = left ? L.B1 : R.B1, JB2 = left ? L.B2 : R.B2;
-  (void) J;
   const float v0 = left ? e.l.v0 : e.r.v0, v1 = left ? e.l.v1 : e.r.v1, v2 = left ? e.l.v2 : e.r.v2;
   const float b1 = left ? e.l.b1 : e.r.b1, b2 = left ? e.l.b2 : e.r.b2, ia = left ? e.l.ia : e.r.ia;
   const float K0 = left ? e.l.K0 : e.r.K0;
@@ -278,62 +393,6 @@ __device__ __forceinline__ int hlld_flux32(const HlldSide32 &L, const HlldSide32
   return 0;
 }
 
-// Total pressure of the HLL state, the first pressure guess, by the Anton et al. 2-D Newton in
-// FP32 from (Z, W) of the average face state, to a step of 1e-6 (the guess only seeds the
-// secants, and is kept in FP32): U as D, E, S0..S2, Bx, B1, B2.  Non-zero when the state fails
-// check_cons, Newton does not converge in 32 iterations, or the primitives fail check_prim;
-// the caller then takes the FP64 ladder.
-__device__ __forceinline__ int hll_pressure32(float gamma, float pfloor, float D, float E, float S0, float S1,
-                                              float S2_, float Bx, float B1, float B2_, float Z, float W, float &pt,
-                                              int &iters)
-{
-  iters = 0;
-  if (!(D >= 0.f) || !(E - D >= 0.f)) return 1;
-  const float gamf = (gamma - 1.f) / gamma;
-  const float S2 = S0 * S0 + S1 * S1 + S2_ * S2_;
-  const float B2 = Bx * Bx + B1 * B1 + B2_ * B2_;
-  const float BS = Bx * S0 + B1 * S1 + B2_ * S2_;
-  const float BS2 = BS * BS;
-  const float iD = 1.f / D;
-  float iW = 1.f / W, iZ = 1.f / Z;
-#pragma unroll 1
-  for (;;) {
-    const float W2 = W * W, iW2 = iW * iW, iW3 = iW2 * iW, iZ2 = iZ * iZ, iZ3 = iZ2 * iZ;
-    const float T = BS2 * iZ2;
-    const float BZ = B2 + Z, u2 = (W2 - 1.f) * iW2;
-    const float Pre = (Z * iW2 - D * iW) * gamf;
-    const float f0Z = 2.f * BZ * (BS2 * iZ3 + u2);
-    const float f0W = 2.f * BZ * BZ * iW3;
-    const float f1Z = 1.f + BS2 * iZ3 - gamf * iW2;
-    const float f1W = (B2 + (2.f * Z - D * W) * gamf) * iW3;
-    const float f0 = BZ * BZ * u2 - (2.f * Z + B2) * T - S2;
-    const float f1 = Z + B2 - E - Pre - 0.5f * B2 * iW2 - 0.5f * T;
-    const float idet = 1.f / (f0Z * f1W - f0W * f1Z);
-    const float dZ = -(f1W * f0 - f0W * f1) * idet;
-    const float dW = -(f0Z * f1 - f1Z * f0) * idet;
-    const float Zn = fabsf(Z + dZ);
-    Z = (Zn < 1e20f) ? Zn : Z;
-    W = fminf(fmaxf(W + dW, 1.f), 1e12f);
-    iZ = 1.f / Z;
-    iW = 1.f / W;
-    const float err = fabsf(dZ * iZ) + fabsf(dW * iW);
-    ++iters;
-    if (!(err > 1e-6f)) {
-      if (!(err == err)) return 1;
-      break;
-    }
-    if (iters == 32) return 1;
-  }
-  const float r = D * iW;
-  float p = r * (Z * iD * iW - 1.f) * gamf;
-  if (pfloor > 0.f && p < pfloor) p = pfloor;
-  const float vB = BS * iZ, iZB = 1.f / (Z + B2);
-  const float v2 = (S2 + vB * (2.f * BS + vB * B2)) * iZB * iZB;
-  if (!(v2 < 1.f) || !(p >= 0.f) || !(r >= 0.f)) return 1;
-  pt = p + 0.5f * (B2 * (1.f - v2) + vB * vB);
-  return 0;
-}
-
 // The FP64 form of the same, for the faces where FP32 does not converge: Newton from the
 // average face state, then the reference's ladder.  Out of line (rare, and its FP64 state
 // would set the register budget of the sweeps).
@@ -365,60 +424,35 @@ static __device__ __noinline__ HllPressure64 hll_pressure64(PhysParams pp, HllSt
   return o;
 }
 
-// HlldRmhdRiemannSolver::IntercellFlux at s = 0 in FP32 (riemann_hlld-rmhd.cpp:179-313).  `src`
-// gives the two face states (reference component order) again where a rare path needs them, so
-// that they need not stay live through the pressure iteration.  Returns 1 when a face state is
+// HlldRmhdRiemannSolver::IntercellFlux at s = 0 in FP32 (riemann_hlld-rmhd.cpp:179-313).  pl, pr
+// and the flux f are in the normal frame of dim.  `src` gives the two face states (reference
+// component order) again where a rare path needs them, so that they need not stay live through
+// the pressure iteration.  Returns 1 when a face state is
 // unphysical (the caller retries with the zone states); used_hllc reports the fallback.
-template <int dim, class Src>
-__device__ __forceinline__ int riemann_hlld32(const PhysParams &pp, const float *pl, const float *pr, float *f,
-                                              float &ml, int &used_hllc, C2PTally *tally, const Src &src)
+template <class Src>
+__device__ __forceinline__ int riemann_hlld32(const PhysParams &pp, int dim, const float *pl, const float *pr,
+                                              float *f, float &ml, int &used_hllc, C2PTally *tally, const Src &src)
 {
   using Tol = RmhdTol<float>;
-  using M = DimMap<dim>;
-  constexpr int B1 = M::B1, B2 = M::B2, B3 = M::B3, S1 = M::S1, S2 = M::S2, S3 = M::S3;
-  constexpr int v1 = M::v1, v2 = M::v2, v3 = M::v3;
   const float gamma = float(pp.gamma), rh_p = gamma / (gamma - 1.f);
-  const float bx = 0.5f * (pl[B1] + pr[B1]);
+  const float bx = 0.5f * (pl[Bx] + pr[Bx]);
   used_hllc = 0;
   if (tally) { tally->iters = 0; tally->attempts = 0; }
   SideState s, t;
-  FastPair fl, fr;
-  if (side_state(gamma, rh_p, pl[rho], pl[pre], pl[v1], pl[v2], pl[v3], bx, pl[B2], pl[B3], s, fl, nullptr)) return 1;
-  if (side_state(gamma, rh_p, pr[rho], pr[pre], pr[v1], pr[v2], pr[v3], bx, pr[B2], pr[B3], t, fr, &fl)) return 1;
-  float ap = fmaxf(fl.hi, fr.hi), am = fminf(fl.lo, fr.lo);
-  if (!(ap <= 1.f && am >= -1.f)) {
-    ap = 1.f;
-    am = -1.f;
-  }
-  ml = fmaxf(ml, fmaxf(fabsf(ap), fabsf(am)));
+  float ap, am;
+  if (face_sides(gamma, pl, pr, bx, s, t, ap, am, ml)) return 1;
   // (Z, W) of the average face state
   float Z0, W0;
   bool usable;
   {
     const float ar = 0.5f * (pl[rho] + pr[rho]), apr = 0.5f * (pl[pre] + pr[pre]);
-    const float a1 = 0.5f * (pl[v1] + pr[v1]), a2 = 0.5f * (pl[v2] + pr[v2]), a3 = 0.5f * (pl[v3] + pr[v3]);
+    const float a1 = 0.5f * (pl[vx] + pr[vx]), a2 = 0.5f * (pl[vy] + pr[vy]), a3 = 0.5f * (pl[vz] + pr[vz]);
     const float i2 = 1.f - (a1 * a1 + a2 * a2 + a3 * a3);
     usable = i2 > 0.f && ar > 0.f && apr > 0.f;
     W0 = rsqrtf(i2);
     Z0 = (ar + rh_p * apr) * W0 * W0;
   }
-  HlldSide32 L, R;
-  L.lam = am;
-  L.D = am * s.D - s.FD;
-  L.E = am * s.E - s.S0;
-  L.m0 = am * s.S0 - s.FS0;
-  L.m1 = am * s.S1 - s.FS1;
-  L.m2 = am * s.S2 - s.FS2;
-  L.B1 = am * s.B1 - s.FB1;
-  L.B2 = am * s.B2 - s.FB2;
-  R.lam = ap;
-  R.D = ap * t.D - t.FD;
-  R.E = ap * t.E - t.S0;
-  R.m0 = ap * t.S0 - t.FS0;
-  R.m1 = ap * t.S1 - t.FS1;
-  R.m2 = ap * t.S2 - t.FS2;
-  R.B1 = ap * t.B1 - t.FB1;
-  R.B2 = ap * t.B2 - t.FB2;
+  const HlldSide32 L = side_jump(s, am), R = side_jump(t, ap);
   float p0 = 0.f;
   int failed;
   {
@@ -434,12 +468,9 @@ __device__ __forceinline__ int riemann_hlld32(const PhysParams &pp, const float 
       HllState32 h;
       h.U[ddd] = D; h.U[tau] = E - D; h.U[Sx] = m0; h.U[Sy] = m1; h.U[Sz] = m2;
       h.U[Bx] = bx; h.U[By] = b1; h.U[Bz] = b2;
-      h.P[rho] = 0.5f * (ql[rho] + qr[rho]);
-      h.P[pre] = 0.5f * (ql[pre] + qr[pre]);
-      h.P[vx] = 0.5f * (ql[v1] + qr[v1]);
-      h.P[vy] = 0.5f * (ql[v2] + qr[v2]);
-      h.P[vz] = 0.5f * (ql[v3] + qr[v3]);
-      h.P[Bx] = bx; h.P[By] = 0.5f * (ql[B2] + qr[B2]); h.P[Bz] = 0.5f * (ql[B3] + qr[B3]);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) h.P[i] = 0.5f * (ql[frame_slot(dim, i)] + qr[frame_slot(dim, i)]);
+      h.P[Bx] = bx;
       const HllPressure64 o = hll_pressure64(pp, h);
       failed = o.err;
       p0 = o.pt;
@@ -466,18 +497,16 @@ __device__ __forceinline__ int riemann_hlld32(const PhysParams &pp, const float 
         SideState o;
         FastPair fp;
         const float *q = left ? ql : qr;
-        side_state(gamma, rh_p, q[rho], q[pre], q[v1], q[v2], q[v3], bx, q[B2], q[B3], o, fp, nullptr);
+        const auto at = [&](int k) { return q[frame_slot(dim, k)]; };
+        side_state(gamma, rh_p, q[rho], q[pre], at(vx), at(vy), at(vz), bx, at(By), at(Bz), o, fp, nullptr);
         U[0] = o.D; U[1] = o.E; U[2] = o.S0; U[3] = o.S1; U[4] = o.S2; U[5] = o.B1; U[6] = o.B2;
       };
       if (hlld_root32(L, R, bx, direct, p, e) == 0 && hlld_flux32(L, R, bx, p, e, F, outer) == 0) {
-        f[ddd] = F[0];
-        f[tau] = F[1];
-        f[S1] = F[2];
-        f[S2] = F[3];
-        f[S3] = F[4];
-        f[B1] = 0.f;
-        f[B2] = F[5];
-        f[B3] = F[6];
+#pragma unroll
+        for (int i = 0; i < 5; ++i) f[i] = F[i];
+        f[Bx] = 0.f;
+        f[By] = F[5];
+        f[Bz] = F[6];
         return 0;
       }
       if (direct) break;
@@ -486,7 +515,7 @@ __device__ __forceinline__ int riemann_hlld32(const PhysParams &pp, const float 
   used_hllc = 1;
   Face8<float> a, b;
   src(a.v, b.v);
-  const HllcOut<float> o = riemann_hllc_fallback<float, dim>(gamma, a, b, ml);
+  const HllcOut<float> o = riemann_hllc32_fallback(dim, gamma, a, b, ml);
   ml = o.ml;
 #pragma unroll
   for (int i = 0; i < 8; ++i) f[i] = o.F[i];

@@ -45,19 +45,22 @@ inline void launch_learned_c2p(const Grid &g, cudaStream_t st, StateCPtr<T> U, T
 
 namespace mgpu {
 
-// One sweep: the flux kernel for (sweep direction, Riemann solver), both compile-time.
+// The flux sweeps of every direction (k_flux), the Riemann solver compile-time; faces[d] faces of
+// direction d + 1.
 template <class T>
-inline void launch_flux(const Grid &g, int d, int rs, unsigned grid, unsigned blk, cudaStream_t st, const T *PA,
-                        T *F, const PhysParams &pp, Ctl *ctl, int s)
+inline void launch_flux(const Grid &g, int rs, const long long *faces, cudaStream_t st, const T *PA, void *const *F,
+                        const PhysParams &pp, Ctl *ctl, int s)
 {
-#define MGPU_FLUX_CASE(D, R)                                                            \
-  if (d == D && rs == R) {                                                              \
-    k_flux<T, D, R><<<grid, blk, 0, st>>>(g, PA, F, pp, ctl, s);                        \
-    return;                                                                             \
+  const unsigned blk = 128;
+  unsigned n[3], total = 0;
+  for (int d = 0; d < 3; ++d) n[d] = total += (unsigned) ((faces[d] + blk - 1) / blk);
+  if (total == 0) return;
+#define MGPU_FLUX_CASE(R)                                                                                         \
+  if (rs == R) {                                                                                                  \
+    k_flux<T, R><<<total, blk, 0, st>>>(g, PA, (T *) F[0], (T *) F[1], (T *) F[2], n[0], n[1], pp, ctl, s);       \
+    return;                                                                                                       \
   }
-  MGPU_FLUX_CASE(1, RIEMANN_HLLD) MGPU_FLUX_CASE(2, RIEMANN_HLLD) MGPU_FLUX_CASE(3, RIEMANN_HLLD)
-  MGPU_FLUX_CASE(1, RIEMANN_HLLC) MGPU_FLUX_CASE(2, RIEMANN_HLLC) MGPU_FLUX_CASE(3, RIEMANN_HLLC)
-  MGPU_FLUX_CASE(1, RIEMANN_HLL) MGPU_FLUX_CASE(2, RIEMANN_HLL) MGPU_FLUX_CASE(3, RIEMANN_HLL)
+  MGPU_FLUX_CASE(RIEMANN_HLLD) MGPU_FLUX_CASE(RIEMANN_HLLC) MGPU_FLUX_CASE(RIEMANN_HLL)
 #undef MGPU_FLUX_CASE
 }
 
@@ -145,7 +148,7 @@ inline cudaError_t launch_phase(const AdvanceArgs &A, int phase, int s)
   const T *F = (const T *) b.F[0], *G = (const T *) b.F[1], *H = (const T *) b.F[2];
   const int ns = num_stages(A.rk);
 
-  const unsigned zb = 256, fb = 128;
+  const unsigned zb = 256;
   const unsigned zgrid = (unsigned) ((g.ninterior + zb - 1) / zb);
   LaunchProfiler *pr = A.prof;
 
@@ -192,13 +195,11 @@ inline cudaError_t launch_phase(const AdvanceArgs &A, int phase, int s)
   } else if (phase == PH_FLUX_UPDATE) {
     if (A.godunov)
       launch_ctu_stage<T>(A, s, s == 0 ? StateCPtr<T>{U0.bulk, U0.B} : StateCPtr<T>{U1.bulk, U1.B});
-    for (int d = 1; d <= g.nd && !A.godunov; ++d) {
-      const long long S = g.s[d - 1];
-      const long long nf = g.nz - 5 * S;
-      if (nf <= 0) continue;
-      const unsigned fgrid = (unsigned) ((nf + fb - 1) / fb);
-      ProfScope ps(pr, st, KC_FLUX, nf);
-      launch_flux<T>(g, d, A.pp.riemann, fgrid, fb, st, PA, (T *) b.F[d - 1], A.pp, A.ctl, s);
+    if (!A.godunov) {
+      long long faces[3] = {0, 0, 0}, sum = 0;
+      for (int d = 0; d < g.nd; ++d) sum += faces[d] = std::max(0ll, g.nz - 5 * g.s[d]);
+      ProfScope ps(pr, st, KC_FLUX, sum);
+      launch_flux<T>(g, A.pp.riemann, faces, st, PA, b.F, A.pp, A.ctl, s);
     }
     const StageKind kind = stage_kind(A.rk, s);
     UpdateArgs ua{kind.combine, kind.c};

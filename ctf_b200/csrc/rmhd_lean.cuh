@@ -113,6 +113,7 @@ __global__ void __launch_bounds__(128, flux_minb<RS>()) k_lean_sweep(Grid g, con
   FluxTally ft{0, 0, 0, 0, 0};
   __shared__ T flo[128][5];   // the carried lower-face flux of each thread
   __shared__ T up[8][128];    // the carried upper-face state of the face's lower zone
+  __shared__ T cols[column_entries<T, RS>() * 128];
   if (t < ncol * nchunk) {
     const int chunk = (int) (t / ncol);
     const long long col = t - (long long) chunk * ncol;
@@ -130,7 +131,7 @@ __global__ void __launch_bounds__(128, flux_minb<RS>()) k_lean_sweep(Grid g, con
     T *slot1 = Bf + (long long) bf_slot(dim, Bz) * g.cs;
     {
       T lo[8], hi[8];
-      zone_states<T>(PA, g.cs, S, pp, base + (long long) (m0 - 1) * S, lo, hi);
+      zone_states<T, RS>(g, PA, pp, dim, base + (long long) (m0 - 1) * S, lo, hi);
 #pragma unroll
       for (int q = 0; q < 8; ++q) up[q][threadIdx.x] = hi[q];
     }
@@ -144,13 +145,15 @@ __global__ void __launch_bounds__(128, flux_minb<RS>()) k_lean_sweep(Grid g, con
           if (dim == 1) asm volatile("prefetch.global.L2 [%0];" ::"l"(U0.bulk + q * g.cs + f));
         }
       }
-      T Pl[8], Pr[8], hi[8], Fo[8];
+      T Pl[8], Pr[8], hi[8], Ff[8], Fo[8];
 #pragma unroll
       for (int q = 0; q < 8; ++q) Pl[q] = up[q][threadIdx.x];
-      zone_states<T>(PA, g.cs, S, pp, f + S, Pr, hi);
+      zone_states<T, RS>(g, PA, pp, dim, f + S, Pr, hi);
 #pragma unroll
       for (int q = 0; q < 8; ++q) up[q][threadIdx.x] = hi[q];
-      solve_face<T, dim, RS>(g, PA, pp, f, Pl, Pr, ml, ft, Fo);
+      solve_face<T, RS, true>(g, PA, pp, dim, f, Pl, Pr, ml, ft, Ff, cols + threadIdx.x);
+#pragma unroll
+      for (int q = 0; q < 8; ++q) Fo[face_slot<T, RS>(dim, q)] = Ff[q];
       if (m >= m0 || chunk == 0) {            // the chunk's first face is its neighbour's last
         slot0[f] = Fo[dim == 1 ? By : Bx];
         slot1[f] = Fo[Bz];
@@ -187,6 +190,7 @@ __global__ void __launch_bounds__(128, flux_minb<RS>()) k_lean_sweep_z(Grid g, c
   FluxTally ft{0, 0, 0, 0, 0};
   __shared__ T up[8][128];   // each zone's upper state
   __shared__ T fs[5][128];   // each thread's flux
+  __shared__ T cols[column_entries<T, RS>() * 128];
   T Pl[8], Pr[8];
   long long z = 0;
   int fk = 0;
@@ -204,16 +208,18 @@ __global__ void __launch_bounds__(128, flux_minb<RS>()) k_lean_sweep_z(Grid g, c
       for (int r = 0; r < 5; ++r) asm volatile("prefetch.global.L2 [%0];" ::"l"(U1.bulk + r * g.cs + z - 1));
     }
     T hi[8];
-    zone_states<T>(PA, g.cs, 1, pp, z, Pr, hi);
+    zone_states<T, RS>(g, PA, pp, 3, z, Pr, hi);
 #pragma unroll
     for (int r = 0; r < 8; ++r) up[r][threadIdx.x] = hi[r];
   }
   __syncthreads();
   if (face) {
-    T Fo[8];
+    T Ff[8], Fo[8];
 #pragma unroll
     for (int r = 0; r < 8; ++r) Pl[r] = up[r][threadIdx.x - 1];
-    solve_face<T, 3, RS>(g, PA, pp, z - 1, Pl, Pr, ml, ft, Fo);
+    solve_face<T, RS, true>(g, PA, pp, 3, z - 1, Pl, Pr, ml, ft, Ff, cols + threadIdx.x);
+#pragma unroll
+    for (int r = 0; r < 8; ++r) Fo[face_slot<T, RS>(3, r)] = Ff[r];
     if (threadIdx.x > 1 || blockIdx.x == 0) {
       Bf[(long long) bf_slot(3, Bx) * g.cs + z - 1] = Fo[Bx];
       Bf[(long long) bf_slot(3, By) * g.cs + z - 1] = Fo[By];
@@ -363,19 +369,23 @@ __global__ void k_lean_download(Grid g, double *__restrict__ aos, long long z0, 
 
 // ---- launch sequence ---------------------------------------------------------------------------
 // Chunk length of a marching sweep over ncol columns of n zones: every chunk costs one face
-// more than its zones, and the launch takes ceil(threads / resident threads) waves of
-// chunk + 1 faces each, so pick the length in [16, 64] that minimises their product.
+// more than its zones (and the reconstruction of one zone more, a quarter of a face), and the
+// launch takes ceil(threads / resident threads) waves of chunks, so pick the length in [2, 64]
+// that minimises their product, a shorter chunk only where it is 5% better (it repeats more
+// faces, which the count of waves does not see).  Large boxes take long chunks, boxes that do
+// not fill the device short ones: there a sweep lasts as long as one thread's chunk
+// (47 x 61 x 53 WENO5 sweeps per RK3 step, 16 zones at least: 0.90 ms; 2 at least: 0.41 ms).
 inline int lean_chunk(long long ncol, int n, long long resident_threads)
 {
-  int best = 32;
+  int best = 64;
   double best_cost = 1e300;
-  for (int L = 16; L <= 64; ++L) {
+  for (int L = 64; L >= 2; --L) {
     const long long nchunk = (n + L - 1) / L;
     const long long Lr = (n + nchunk - 1) / nchunk;   // the longest chunk with this count
     if (Lr != L) continue;
     const long long threads = ncol * nchunk;
-    const double cost = (double) ((threads + resident_threads - 1) / resident_threads) * (double) (L + 1);
-    if (cost < best_cost) {
+    const double cost = (double) ((threads + resident_threads - 1) / resident_threads) * (L + 1.25);
+    if (cost < 0.95 * best_cost) {
       best_cost = cost;
       best = L;
     }

@@ -37,7 +37,6 @@ template <> struct RmhdTol<double> {
   static constexpr double contact = 1e-8;       // UnmatchedContactSpeed
   static constexpr double degenerate = 1e-8;    // |am - aL.v| etc.
   static constexpr double bx_small = 1e-8;      // |Bx| < 1e-8 -> eq. (55) guess only
-  static constexpr double bjump = 1e-12;        // JumpInNormalBfield
   static constexpr double hllc_bx = 1e-12;      // SMALL_BX
   static constexpr double hllc_a = 1e-10;       // SMALL_A
 };
@@ -50,7 +49,6 @@ template <> struct RmhdTol<float> {
   static constexpr float contact = 2e-4f;
   static constexpr float degenerate = 1e-6f;
   static constexpr float bx_small = 1e-6f;
-  static constexpr float bjump = 1e-6f;
 #ifdef MGPU_HLLC_BX_F32
   static constexpr float hllc_bx = MGPU_HLLC_BX_F32;
 #else
@@ -63,7 +61,9 @@ __device__ __forceinline__ double m_sqrt(double x) { return sqrt(x); }
 __device__ __forceinline__ float m_sqrt(float x) { return sqrtf(x); }
 __device__ __forceinline__ double m_abs(double x) { return fabs(x); }
 __device__ __forceinline__ float m_abs(float x) { return fabsf(x); }
-__device__ __forceinline__ double m_cbrt_pow(double x) { return pow(x, 1. / 3.); }
+// out of line: the one-real-root branch of the resolvent cubic is rare (no face of the turbulence
+// states, 0.4% of the stress box's)
+static __device__ __noinline__ double m_cbrt_pow(double x) { return pow(x, 1. / 3.); }
 __device__ __forceinline__ float m_cbrt_pow(float x) { return cbrtf(x); }
 __device__ __forceinline__ double m_acos(double x) { return acos(x); }
 __device__ __forceinline__ float m_acos(float x) { return acosf(x); }
@@ -72,8 +72,24 @@ __device__ __forceinline__ float m_cos(float x) { return cosf(x); }
 __device__ __forceinline__ double m_sin(double x) { return sin(x); }
 __device__ __forceinline__ float m_sin(float x) { return sinf(x); }
 
+// Division by a denominator that several quotients share.  FP64: the correctly rounded quotient
+// from the correctly rounded reciprocal and one exact remainder (Markstein, IBM J. Res. Dev.
+// 34, 1990) -- the value a / b has, in three operations instead of a division's ten or so.  A
+// non-finite quotient may come out as NaN instead of infinity.  FP32 multiplies by the
+// reciprocal, as its fast division does.
+template <class T> struct Recip {
+  T b, r;
+};
+template <class T> __device__ __forceinline__ Recip<T> recip(T b) { return {b, T(1) / b}; }
+__device__ __forceinline__ double operator/(double a, const Recip<double> &d)
+{
+  const double q = a * d.r;
+  return fma(fma(-q, d.b, a), d.r, q);
+}
+__device__ __forceinline__ float operator/(float a, const Recip<float> &d) { return a * d.r; }
+
 // ---- EOS (Mara/eos.cpp:13-29) -------------------------------------------------------
-template <class T> __device__ __forceinline__ T eos_internal(T gamma, T p) { return p / (gamma - 1); }
+template <class T> __device__ __forceinline__ T eos_internal(T gamma, T p) { return p / recip(gamma - 1); }
 template <class T> __device__ __forceinline__ T eos_cs2(T gamma, T r, T p)
 {
   const T rhoh = r + eos_internal(gamma, p) + p;
@@ -100,15 +116,16 @@ __device__ __forceinline__ int prim_to_cons(T gamma, const T *P, T *U)
   const T Bv = P[Bx] * P[vx] + P[By] * P[vy] + P[Bz] * P[vz];
   const T W2 = T(1) / (T(1) - V2);
   const T W = m_sqrt(W2);
+  const Recip<T> iW = recip(W), ir = recip(P[rho]);
   const T b0 = W * Bv;
   const T b2 = (B2 + b0 * b0) / W2;
-  const T bx = (P[Bx] + b0 * W * P[vx]) / W;
-  const T by = (P[By] + b0 * W * P[vy]) / W;
-  const T bz = (P[Bz] + b0 * W * P[vz]) / W;
-  const T e = eos_internal(gamma, P[pre]) / P[rho];
-  const T e_ = e + T(0.5) * b2 / P[rho];
+  const T bx = (P[Bx] + b0 * W * P[vx]) / iW;
+  const T by = (P[By] + b0 * W * P[vy]) / iW;
+  const T bz = (P[Bz] + b0 * W * P[vz]) / iW;
+  const T e = eos_internal(gamma, P[pre]) / ir;
+  const T e_ = e + T(0.5) * b2 / ir;
   const T p_ = P[pre] + T(0.5) * b2;
-  const T h_ = T(1) + e_ + p_ / P[rho];
+  const T h_ = T(1) + e_ + p_ / ir;
   U[ddd] = P[rho] * W;
   U[tau] = P[rho] * h_ * W2 - p_ - b0 * b0 - U[ddd];
   U[Sx] = P[rho] * h_ * W2 * P[vx] - b0 * bx;
@@ -122,34 +139,42 @@ __device__ __forceinline__ int prim_to_cons(T gamma, const T *P, T *U)
 }
 
 // ---- quartic (Mara/quartic.cpp:28-148) -------------------------------------------------
+// x1 and the largest of the others (x3) of x^3 + c2 x^2 + c1 x + c0, as the quartic uses them; nr
+// real roots (Mara/quartic.cpp:28-80).
 template <class T>
-__device__ __forceinline__ void cubic(T c2, T c1, T c0, T &x1, T &x2, T &x3, int &nr)
+__device__ __forceinline__ void cubic(T c2, T c1, T c0, T &x1, T &x3, int &nr)
 {
   // c3 = 1: the reference divides by it, which is exact.
   const T a2 = c2, a1 = c1, a0 = c0;
-  const T q = a1 / T(3) - a2 * a2 / T(9);
-  const T r = (a1 * a2 - T(3) * a0) / T(6) - a2 * a2 * a2 / T(27);
+  const Recip<T> i3 = recip(T(3));
+  const T q = a1 / i3 - a2 * a2 / recip(T(9));
+  const T r = (a1 * a2 - T(3) * a0) / recip(T(6)) - a2 * a2 * a2 / recip(T(27));
   const T delta = q * q * q + r * r;
   if (delta > T(0)) {
     T s1 = r + m_sqrt(delta);
     s1 = (s1 >= T(0)) ? m_cbrt_pow(s1) : -m_cbrt_pow(-s1);
     T s2 = r - m_sqrt(delta);
     s2 = (s2 >= T(0)) ? m_cbrt_pow(s2) : -m_cbrt_pow(-s2);
-    x1 = (s1 + s2) - a2 / T(3);
-    x2 = x3 = T(-0.5) * (s1 + s2) - a2 / T(3);
+    x1 = (s1 + s2) - a2 / i3;
+    x3 = T(-0.5) * (s1 + s2) - a2 / i3;
     nr = 1;
   } else if (delta < T(0)) {
-    const T theta = m_acos(r / m_sqrt(-q * q * q)) / T(3);
-    const T costh = m_cos(theta), sinth = m_sin(theta), sq = m_sqrt(-q);
-    const T sqrt3 = T(1.7320508075688772);
-    x1 = T(2) * sq * costh - a2 / T(3);
-    x2 = -sq * costh - a2 / T(3) - sqrt3 * sq * sinth;
-    x3 = -sq * costh - a2 / T(3) + sqrt3 * sq * sinth;
+    const T theta = m_acos(r / m_sqrt(-q * q * q)) / i3;
+    const T costh = m_cos(theta), sq = m_sqrt(-q);
+    x1 = T(2) * sq * costh - a2 / i3;
+    // theta is in [0, pi/3], where 2 cos >= sqrt(3) sin - cos: x1 is the largest root, and only
+    // next to pi/3 (cos = 1/2) can rounding put x3 above it
+    x3 = x1;
+    if (!(costh > T(0.5001))) {
+      const T sinth = m_sin(theta);
+      const T sqrt3 = T(1.7320508075688772);
+      x3 = -sq * costh - a2 / i3 + sqrt3 * sq * sinth;
+    }
     nr = 3;
   } else {
     const T s = (r >= T(0)) ? m_cbrt_pow(r) : -m_cbrt_pow(-r);
-    x1 = T(2) * s - a2 / T(3);
-    x2 = x3 = -s - a2 / T(3);
+    x1 = T(2) * s - a2 / i3;
+    x3 = -s - a2 / i3;
     nr = 3;
   }
 }
@@ -159,13 +184,14 @@ __device__ __forceinline__ void cubic(T c2, T c1, T c0, T &x1, T &x2, T &x3, int
 template <class T>
 __device__ __forceinline__ void quartic_extreme_roots(T d4, T d3, T d2, T d1, T d0, T &ap, T &am)
 {
-  const T a3 = d3 / d4, a2 = d2 / d4, a1 = d1 / d4, a0 = d0 / d4;
+  const Recip<T> i4 = recip(d4);
+  const T a3 = d3 / i4, a2 = d2 / i4, a1 = d1 / i4, a0 = d0 / i4;
   const T au2 = -a2;
   const T au1 = (a1 * a3 - T(4) * a0);
   const T au0 = T(4) * a0 * a2 - a1 * a1 - a0 * a3 * a3;
-  T x1, x2, x3;
+  T x1, x3;
   int nr;
-  cubic<T>(au2, au1, au0, x1, x2, x3, nr);
+  cubic<T>(au2, au1, au0, x1, x3, nr);
   const T u1 = (nr == 1) ? x1 : ((x1 > x3) ? x1 : x3);
   const T R2 = T(0.25) * a3 * a3 + u1 - a2;
   const T R = (R2 > T(0)) ? m_sqrt(R2) : T(0);
@@ -291,21 +317,22 @@ __device__ __forceinline__ void flux_and_eigenvalues(T gamma, const T *U, const 
   const T Bv = P[Bx] * P[vx] + P[By] * P[vy] + P[Bz] * P[vz];
   const T W2 = T(1) / (T(1) - V2);
   const T W = m_sqrt(W2);
+  const Recip<T> iW = recip(W), ir = recip(P[rho]);
   const T b0 = W * Bv;
   const T b2 = (B2 + b0 * b0) / W2;
-  const T bx = (P[Bx] + b0 * W * P[vx]) / W;
-  const T by = (P[By] + b0 * W * P[vy]) / W;
-  const T bz = (P[Bz] + b0 * W * P[vz]) / W;
-  const T e = eos_internal(gamma, P[pre]) / P[rho];
+  const T bx = (P[Bx] + b0 * W * P[vx]) / iW;
+  const T by = (P[By] + b0 * W * P[vy]) / iW;
+  const T bz = (P[Bz] + b0 * W * P[vz]) / iW;
+  const T e = eos_internal(gamma, P[pre]) / ir;
   const T p_ = P[pre] + T(0.5) * b2;
-  const T h = T(1) + e + P[pre] / P[rho];
+  const T h = T(1) + e + P[pre] / ir;
   T vi, bi;
   if (dim == 1) {
     F[ddd] = U[ddd] * P[vx];
-    F[tau] = U[tau] * P[vx] - b0 * P[Bx] / W + p_ * P[vx];
-    F[Sx] = U[Sx] * P[vx] - bx * P[Bx] / W + p_;
-    F[Sy] = U[Sy] * P[vx] - by * P[Bx] / W;
-    F[Sz] = U[Sz] * P[vx] - bz * P[Bx] / W;
+    F[tau] = U[tau] * P[vx] - b0 * P[Bx] / iW + p_ * P[vx];
+    F[Sx] = U[Sx] * P[vx] - bx * P[Bx] / iW + p_;
+    F[Sy] = U[Sy] * P[vx] - by * P[Bx] / iW;
+    F[Sz] = U[Sz] * P[vx] - bz * P[Bx] / iW;
     F[Bx] = T(0);
     F[By] = P[vx] * P[By] - P[vy] * P[Bx];
     F[Bz] = P[vx] * P[Bz] - P[vz] * P[Bx];
@@ -313,10 +340,10 @@ __device__ __forceinline__ void flux_and_eigenvalues(T gamma, const T *U, const 
     bi = bx;
   } else if (dim == 2) {
     F[ddd] = U[ddd] * P[vy];
-    F[tau] = U[tau] * P[vy] - b0 * P[By] / W + p_ * P[vy];
-    F[Sx] = U[Sx] * P[vy] - bx * P[By] / W;
-    F[Sy] = U[Sy] * P[vy] - by * P[By] / W + p_;
-    F[Sz] = U[Sz] * P[vy] - bz * P[By] / W;
+    F[tau] = U[tau] * P[vy] - b0 * P[By] / iW + p_ * P[vy];
+    F[Sx] = U[Sx] * P[vy] - bx * P[By] / iW;
+    F[Sy] = U[Sy] * P[vy] - by * P[By] / iW + p_;
+    F[Sz] = U[Sz] * P[vy] - bz * P[By] / iW;
     F[Bx] = P[vy] * P[Bx] - P[vx] * P[By];
     F[By] = T(0);
     F[Bz] = P[vy] * P[Bz] - P[vz] * P[By];
@@ -324,10 +351,10 @@ __device__ __forceinline__ void flux_and_eigenvalues(T gamma, const T *U, const 
     bi = by;
   } else {
     F[ddd] = U[ddd] * P[vz];
-    F[tau] = U[tau] * P[vz] - b0 * P[Bz] / W + p_ * P[vz];
-    F[Sx] = U[Sx] * P[vz] - bx * P[Bz] / W;
-    F[Sy] = U[Sy] * P[vz] - by * P[Bz] / W;
-    F[Sz] = U[Sz] * P[vz] - bz * P[Bz] / W + p_;
+    F[tau] = U[tau] * P[vz] - b0 * P[Bz] / iW + p_ * P[vz];
+    F[Sx] = U[Sx] * P[vz] - bx * P[Bz] / iW;
+    F[Sy] = U[Sy] * P[vz] - by * P[Bz] / iW;
+    F[Sz] = U[Sz] * P[vz] - bz * P[Bz] / iW + p_;
     F[Bx] = P[vz] * P[Bx] - P[vx] * P[Bz];
     F[By] = P[vz] * P[By] - P[vy] * P[Bz];
     F[Bz] = T(0);
@@ -357,8 +384,9 @@ __device__ __forceinline__ void flux_and_eigenvalues(T gamma, const T *U, const 
   }
   const T cs2 = eos_cs2(gamma, P[rho], P[pre]);
   const T W4 = W2 * W2, v2 = vi * vi, v3 = vi * v2, v4 = vi * v3;
-  const T K = P[rho] * h * (T(1) / cs2 - T(1)) * W4;
-  const T L = -(P[rho] * h + b2 / cs2) * W2;
+  const Recip<T> ics = recip(cs2);
+  const T K = P[rho] * h * (ics.r - T(1)) * W4;
+  const T L = -(P[rho] * h + b2 / ics) * W2;
   const T A4 = K - L - b0 * b0;
   const T A3 = T(-4) * K * vi + L * vi * T(2) + T(2) * b0 * bi;
   const T A2 = T(6) * K * v2 + L * (T(1) - v2) + b0 * b0 - bi * bi;
@@ -417,12 +445,13 @@ __device__ __forceinline__ int check_prim(const T *P)
 __device__ __forceinline__ int c2p_reconstruct(const C2PState &s, double Z, double W, double *Pout)
 {
   double P[8];
+  const Recip<double> iW = recip(W), iZB = recip(Z + s.B2);
   const double b0 = s.BS * W / Z;
-  P[rho] = s.D / W;
-  P[pre] = (s.D / W) * (Z / (s.D * W) - 1.0) * s.gamf;
-  P[vx] = (s.Sxyz[0] + b0 * s.Bxyz[0] / W) / (Z + s.B2);
-  P[vy] = (s.Sxyz[1] + b0 * s.Bxyz[1] / W) / (Z + s.B2);
-  P[vz] = (s.Sxyz[2] + b0 * s.Bxyz[2] / W) / (Z + s.B2);
+  P[rho] = s.D / iW;
+  P[pre] = (s.D / iW) * (Z / (s.D * W) - 1.0) * s.gamf;
+  P[vx] = (s.Sxyz[0] + b0 * s.Bxyz[0] / iW) / iZB;
+  P[vy] = (s.Sxyz[1] + b0 * s.Bxyz[1] / iW) / iZB;
+  P[vz] = (s.Sxyz[2] + b0 * s.Bxyz[2] / iW) / iZB;
   P[Bx] = s.Bxyz[0];
   P[By] = s.Bxyz[1];
   P[Bz] = s.Bxyz[2];
@@ -465,17 +494,19 @@ __device__ __forceinline__ int c2p_anton2dzw(const C2PState &s, double Z, double
   const double D = s.D, B2 = s.B2, BS2 = s.BS2, S2 = s.S2, gamf = s.gamf, Tau = s.Tau;
   double error = 1.0;
   iters = 0;
+  Recip<double> iW = recip(W);
   while (error > 1e-12) {
     const double Z2 = Z * Z, Z3 = Z * Z2, W2 = W * W, W3 = W * W2;
-    const double Pre = (D / W) * (Z / (D * W) - 1.0) * gamf;
+    const Recip<double> iW2 = recip(W2), iW3 = recip(W3), iZ2 = recip(Z2);
+    const double Pre = (D / iW) * (Z / (D * W) - 1.0) * gamf;
     const double df0dZ = 2 * (B2 + Z) * (BS2 * W2 + (W2 - 1) * Z3) / (W2 * Z3);
-    const double df0dW = 2 * (B2 + Z) * (B2 + Z) / W3;
-    const double df1dZ = 1.0 + BS2 / Z3 - gamf / W2;
-    const double df1dW = B2 / W3 + (2 * Z - D * W) / W3 * gamf;
-    const double f0 = -S2 + (Z + B2) * (Z + B2) * (W2 - 1) / W2 - (2 * Z + B2) * BS2 / Z2;
-    const double f1 = -Tau + Z + B2 - Pre - 0.5 * B2 / W2 - 0.5 * BS2 / Z2 - D;
-    const double det = df0dZ * df1dW - df0dW * df1dZ;
-    const double G0 = df1dW / det, G1 = -df0dW / det, G2 = -df1dZ / det, G3 = df0dZ / det;
+    const double df0dW = 2 * (B2 + Z) * (B2 + Z) / iW3;
+    const double df1dZ = 1.0 + BS2 / Z3 - gamf / iW2;
+    const double df1dW = B2 / iW3 + (2 * Z - D * W) / iW3 * gamf;
+    const double f0 = -S2 + (Z + B2) * (Z + B2) * (W2 - 1) / iW2 - (2 * Z + B2) * BS2 / iZ2;
+    const double f1 = -Tau + Z + B2 - Pre - 0.5 * B2 / iW2 - 0.5 * BS2 / iZ2 - D;
+    const Recip<double> idet = recip(df0dZ * df1dW - df0dW * df1dZ);
+    const double G0 = df1dW / idet, G1 = -df0dW / idet, G2 = -df1dZ / idet, G3 = df0dZ / idet;
     const double dZ = -(G0 * f0 + G1 * f1);
     const double dW = -(G2 * f0 + G3 * f1);
     double Zn = Z + dZ, Wn = W + dW;
@@ -485,7 +516,8 @@ __device__ __forceinline__ int c2p_anton2dzw(const C2PState &s, double Z, double
     Wn = (Wn < 1e12) ? Wn : 1e12;
     Z = Zn;
     W = Wn;
-    error = fabs(dZ / Z) + fabs(dW / W);
+    iW = recip(W);
+    error = fabs(dZ / Z) + fabs(dW / iW);
     if (++iters == 250) return C2P_MAXITER;
   }
   return c2p_reconstruct(s, Z, W, P);
@@ -919,6 +951,7 @@ __device__ __forceinline__ int riemann_hll(T gamma, const T *Pl, const T *Pr, T 
     if (s <= am) F[i] = Fl[i];
     else if (am < s && s <= ap) F[i] = Fh;
     else if (ap < s) F[i] = Fr[i];
+    else F[i] = T(0);   // unordered (NaN) speeds: the reference's zeroed flux stays
   }
   return 0;
 }
@@ -939,14 +972,10 @@ __device__ __forceinline__ T hllc_contact_speed(T a, T b, T c)
 }
 
 // The HLL average, the HLLC star states and the flux at s = 0 from the two sides' states,
-// fluxes (total-energy convention) and the outer speeds.  `safeguard` (the FP32 path): a
-// non-finite contact speed or star state -- which FP32 overflow or a vanishing FP32
-// denominator can produce where FP64 stays finite -- takes the HLL flux instead.  Star
-// states that are merely unphysical (negative pressure, superluminal contact) are kept, as
-// the reference keeps them, so the two precisions take the same branch.
+// fluxes (total-energy convention) and the outer speeds (FP64; FP32 faces take riemann_hllc32).
 template <class C, int dim>
 __device__ __forceinline__ void hllc_star_flux(const C *Pl, const C *Pr, const C *Ul, const C *Ur, const C *Fl,
-                                               const C *Fr, C ap, C am, C *F, bool safeguard)
+                                               const C *Fr, C ap, C am, C *F)
 {
   using T = C;
   using Tol = RmhdTol<T>;
@@ -958,7 +987,7 @@ __device__ __forceinline__ void hllc_star_flux(const C *Pl, const C *Pr, const C
     Uh[i] = (ap * Ur[i] - am * Ul[i] + (Fl[i] - Fr[i])) / (ap - am);
     Fh[i] = (ap * Fl[i] - am * Fr[i] + ap * am * (Ur[i] - Ul[i])) / (ap - am);
   }
-  T Ul_[8], Ur_[8], lc, hllc_star_p;
+  T Ul_[8], Ur_[8], lc;
   if (m_abs(Uh[B1]) > T(Tol::hllc_bx)) {
     const T BdFB = Uh[B2] * Fh[B2] + Uh[B3] * Fh[B3];
     const T a = Fh[tau] - BdFB;
@@ -972,7 +1001,6 @@ __device__ __forceinline__ void hllc_star_flux(const C *Pl, const C *Pr, const C
     const T vdv = w1 * w1 + w2 * w2 + w3 * w3;
     const T gm2 = T(1) / (T(1) - vdv);
     const T ps = Fh[S1] + b1 * b1 / gm2 - (Fh[tau] - b1 * vdB) * w1;
-    hllc_star_p = ps;
     Ul_[ddd] = (am - Pl[v1]) / (am - w1) * Ul[ddd];
     Ur_[ddd] = (ap - Pr[v1]) / (ap - w1) * Ur[ddd];
     Ul_[tau] = (am * Ul[tau] - Ul[S1] + ps * w1 - vdB * b1) / (am - w1);
@@ -992,7 +1020,6 @@ __device__ __forceinline__ void hllc_star_flux(const C *Pl, const C *Pr, const C
     const T c = Uh[S1];
     const T v1_ = lc = hllc_contact_speed(a, b, c);
     const T p_ = -Fh[tau] * v1_ + Fh[S1];
-    hllc_star_p = p_;
     Ul_[ddd] = (am - Pl[v1]) / (am - v1_) * Ul[ddd];
     Ur_[ddd] = (ap - Pr[v1]) / (ap - v1_) * Ur[ddd];
     Ul_[tau] = (am * Ul[tau] - Ul[S1] + p_ * v1_) / (am - v1_);
@@ -1011,23 +1038,13 @@ __device__ __forceinline__ void hllc_star_flux(const C *Pl, const C *Pr, const C
     Ur_[B3] = (ap - Pr[v1]) / (ap - v1_) * Ur[B3];
   }
   const T s = T(0);
-  if (safeguard) {
-    bool bad = !(isfinite(lc) && isfinite(hllc_star_p));
-#pragma unroll
-    for (int i = 0; i < 8; ++i) bad = bad || !isfinite(Ul_[i]) || !isfinite(Ur_[i]);
-    if (bad) {
-#pragma unroll
-      for (int i = 0; i < 8; ++i) F[i] = (s <= am) ? Fl[i] : (s <= ap ? Fh[i] : Fr[i]);
-      F[tau] -= F[ddd];
-      return;
-    }
-  }
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
     if (s <= am) F[i] = Fl[i];
     else if (am < s && s <= lc) F[i] = Fl[i] + am * (Ul_[i] - Ul[i]);
     else if (lc < s && s <= ap) F[i] = Fr[i] + ap * (Ur_[i] - Ur[i]);
     else if (ap < s) F[i] = Fr[i];
+    else F[i] = T(0);   // unordered (NaN) speeds: the reference's zeroed flux stays
   }
   F[tau] -= F[ddd];
 }
@@ -1053,31 +1070,55 @@ __device__ __forceinline__ int riemann_hllc(T gamma, const T *pl, const T *pr, T
   const T am = (eml < emr) ? eml : emr;
   const T l = face_lambda(ap, am);
   if (ml < l) ml = l;
-  hllc_star_flux<T, dim>(Pl, Pr, Ul, Ur, Fl, Fr, ap, am, F, sizeof(T) < sizeof(double));
+  hllc_star_flux<T, dim>(Pl, Pr, Ul, Ur, Fl, Fr, ap, am, F);
   return 0;
 }
 
+// Component of slot k of a state or flux in the normal frame of direction dim (1..3): density and
+// energy (pressure), then the vector components from the normal one on, cyclically, as the
+// reference's IntercellFlux switch orders them.
+__host__ __device__ constexpr int frame_slot(int dim, int k)
+{
+  return k < 2 ? k : k < 5 ? 2 + (dim - 1 + k - 2) % 3 : 5 + (dim - 1 + k - 5) % 3;
+}
+
 // Out-of-line HLLC for the HLLD fallback (rare): arguments and result by value so that the
-// caller's face states stay in registers on its hot path.
+// caller's face states stay in registers on its hot path.  States in the reference's component
+// order, the flux in the normal frame of dim.
 template <class T> struct Face8 { T v[8]; };
 template <class T> struct HllcOut { T F[8]; T ml; int err; };
-template <class T, int dim>
-static __device__ __noinline__ HllcOut<T> riemann_hllc_fallback(T gamma, Face8<T> pl, Face8<T> pr, T ml)
+template <class T>
+static __device__ __noinline__ HllcOut<T> riemann_hllc_fallback(int dim, T gamma, Face8<T> pl, Face8<T> pr, T ml)
 {
   HllcOut<T> o;
   o.ml = ml;
-  o.err = riemann_hllc<T, dim>(gamma, pl.v, pr.v, o.F, o.ml);
+  T F[8];
+  if (dim == 1) o.err = riemann_hllc<T, 1>(gamma, pl.v, pr.v, F, o.ml);
+  else if (dim == 2) o.err = riemann_hllc<T, 2>(gamma, pl.v, pr.v, F, o.ml);
+  else o.err = riemann_hllc<T, 3>(gamma, pl.v, pr.v, F, o.ml);
+#pragma unroll
+  for (int k = 0; k < 8; ++k) o.F[k] = F[frame_slot(dim, k)];
   return o;
 }
+
+// ---- HLLD (Mignone, Ugliano & Bodo 2009; Mara/riemann_hlld-rmhd.cpp) -------------------------
+// A thread's column of an array of shared memory (entry i at p[i * stride]): the stride is the
+// block's width, so a warp's accesses to one entry are conflict-free.
+template <class T> struct Column {
+  T *p;
+  int stride;
+  __device__ __forceinline__ T &operator[](int i) const { return p[i * stride]; }
+};
 
 // ---- HLLD (Mignone, Ugliano & Bodo 2009; Mara/riemann_hlld-rmhd.cpp) -------------------------
 template <class T> struct HlldJump { T E, D, B[3], m[3]; };
 template <class T> struct HlldInner { T B[3], v[3]; };
 
+// Equation 48: the outer speeds, the normal field (the same on both sides) and the jumps
+// J = lambda U - F across the outer waves (normal frame, total-energy convention tau + D).
 template <class T>
 struct HlldEqn {
-  T Ul[8], Ur[8], Fl[8], Fr[8];   // normal-frame states, total-energy convention (tau + D)
-  T ap, am, PlBx, PrBx;
+  T ap, am, bx;
   HlldJump<T> L, R;
 };
 
@@ -1085,7 +1126,7 @@ template <class T> __device__ __forceinline__ T dot3(const T *v, const T *w) { r
 template <class T> __device__ __forceinline__ T dot1(const T *v) { return v[0] * v[0] + v[1] * v[1] + v[2] * v[2]; }
 
 template <class T>
-__device__ __forceinline__ void hlld_side(const HlldJump<T> &J, T a, T UBx, T p, HlldInner<T> &s)
+__device__ __forceinline__ void hlld_side(const HlldJump<T> &J, T a, T UBx, T p, HlldInner<T> &s, Recip<T> &ia)
 {
   using Tol = RmhdTol<T>;
   const T A = J.m[0] - a * J.E + p * (T(1) - a * a);
@@ -1094,55 +1135,74 @@ __device__ __forceinline__ void hlld_side(const HlldJump<T> &J, T a, T UBx, T p,
   const T Q = -A - G + (UBx * UBx) * (T(1) - a * a);
   T X = UBx * (A * a * UBx + C) - (A + G) * (a * p + J.E);
   if (m_abs(X) < T(Tol::x_small)) X = T(Tol::x_small);
-  s.v[0] = (UBx * (A * UBx + a * C) - (A + G) * (p + J.m[0])) / X;
-  s.v[1] = (Q * J.m[1] + J.B[1] * (C + UBx * (a * J.m[0] - J.E))) / X;
-  s.v[2] = (Q * J.m[2] + J.B[2] * (C + UBx * (a * J.m[0] - J.E))) / X;
-  s.B[0] = (J.B[0] - UBx * s.v[0]) / (a - s.v[0]);
-  s.B[1] = (J.B[1] - UBx * s.v[1]) / (a - s.v[0]);
-  s.B[2] = (J.B[2] - UBx * s.v[2]) / (a - s.v[0]);
+  const Recip<T> iX = recip(X);
+  s.v[0] = (UBx * (A * UBx + a * C) - (A + G) * (p + J.m[0])) / iX;
+  s.v[1] = (Q * J.m[1] + J.B[1] * (C + UBx * (a * J.m[0] - J.E))) / iX;
+  s.v[2] = (Q * J.m[2] + J.B[2] * (C + UBx * (a * J.m[0] - J.E))) / iX;
+  ia = recip(a - s.v[0]);
+  s.B[0] = (J.B[0] - UBx * s.v[0]) / ia;
+  s.B[1] = (J.B[1] - UBx * s.v[1]) / ia;
+  s.B[2] = (J.B[2] - UBx * s.v[2]) / ia;
 }
+
+// The states between the fast waves at total pressure p.
+template <class T> struct HlldFill {
+  T Kl[3], Kr[3], Bc[3], etaL, etaR, wL, wR;
+  HlldInner<T> aL, aR;
+};
 
 // FillInnerWaveStates (riemann_hlld-rmhd.cpp:357-420)
 template <class T>
-__device__ __forceinline__ void hlld_fill(const HlldEqn<T> &q, T p, T *Kl, T *Kr, T *Bc, T &etaL, T &etaR,
-                                          T &wL, T &wR, HlldInner<T> &aL, HlldInner<T> &aR)
+__device__ __forceinline__ void hlld_fill(const HlldEqn<T> &q, T p, HlldFill<T> &f)
 {
   using Tol = RmhdTol<T>;
-  hlld_side(q.L, q.am, q.Ul[Bx], p, aL);
-  hlld_side(q.R, q.ap, q.Ur[Bx], p, aR);
-  wL = p + (q.L.E - dot3(aL.v, q.L.m)) / (q.am - aL.v[0]);
-  wR = p + (q.R.E - dot3(aR.v, q.R.m)) / (q.ap - aR.v[0]);
-  if (wL < T(0)) wL *= T(-1);
-  if (wR < T(0)) wR *= T(-1);
-  etaL = T(-sgn(q.Ul[Bx])) * m_sqrt(wL);
-  etaR = T(+sgn(q.Ur[Bx])) * m_sqrt(wR);
+  HlldInner<T> &aL = f.aL, &aR = f.aR;
+  Recip<T> il, ir;
+  hlld_side(q.L, q.am, q.bx, p, aL, il);
+  hlld_side(q.R, q.ap, q.bx, p, aR, ir);
+  f.wL = p + (q.L.E - dot3(aL.v, q.L.m)) / il;
+  f.wR = p + (q.R.E - dot3(aR.v, q.R.m)) / ir;
+  if (f.wL < T(0)) f.wL *= T(-1);
+  if (f.wR < T(0)) f.wR *= T(-1);
+  f.etaL = T(-sgn(q.bx)) * m_sqrt(f.wL);
+  f.etaR = T(+sgn(q.bx)) * m_sqrt(f.wR);
+  const Recip<T> dl = recip(q.am * p + q.L.E + q.bx * f.etaL), dr = recip(q.ap * p + q.R.E + q.bx * f.etaR);
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
-    Kl[k] = (q.L.m[k] + p * T(k == 0) + q.L.B[k] * etaL) / (q.am * p + q.L.E + q.Ul[Bx] * etaL);
-    Kr[k] = (q.R.m[k] + p * T(k == 0) + q.R.B[k] * etaR) / (q.ap * p + q.R.E + q.Ur[Bx] * etaR);
-    Bc[k] = ((aR.B[k] * (Kr[0] - aR.v[0]) + aR.B[0] * aR.v[k]) -
-             (aL.B[k] * (Kl[0] - aL.v[0]) + aL.B[0] * aL.v[k])) / (Kr[0] - Kl[0]);
-    if (m_abs(Kr[0] - Kl[0]) < T(Tol::k_small)) Bc[k] = T(0);
+    f.Kl[k] = (q.L.m[k] + p * T(k == 0) + q.L.B[k] * f.etaL) / dl;
+    f.Kr[k] = (q.R.m[k] + p * T(k == 0) + q.R.B[k] * f.etaR) / dr;
   }
+  const Recip<T> dk = recip(f.Kr[0] - f.Kl[0]);
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    f.Bc[k] = ((aR.B[k] * (f.Kr[0] - aR.v[0]) + aR.B[0] * aR.v[k]) -
+               (aL.B[k] * (f.Kl[0] - aL.v[0]) + aL.B[0] * aL.v[k])) / dk;
+    if (m_abs(f.Kr[0] - f.Kl[0]) < T(Tol::k_small)) f.Bc[k] = T(0);
+  }
+}
+
+// The residual of eq. 48 from the states at its pressure.
+template <class T>
+__device__ __forceinline__ T hlld_residual(const HlldFill<T> &f)
+{
+  using Tol = RmhdTol<T>;
+  const T delK = f.Kr[0] - f.Kl[0];
+  const T Bch[3] = { f.Bc[0] * delK, f.Bc[1] * delK, f.Bc[2] * delK };
+  const T Yl = (T(1) - dot1(f.Kl)) / (f.etaL * delK - dot3(f.Kl, Bch));
+  const T Yr = (T(1) - dot1(f.Kr)) / (f.etaR * delK - dot3(f.Kr, Bch));
+  if (m_abs(delK) < T(Tol::k_small)) return T(0);
+  if (m_abs(f.Bc[0]) < T(Tol::k_small)) return delK;
+  return delK * (T(1) - f.Bc[0] * (Yr - Yl));
 }
 
 // HlldEquation48::Function (riemann_hlld-rmhd.cpp:422-452); returns non-zero on "throw".
 template <class T>
 __device__ __forceinline__ int hlld_function(const HlldEqn<T> &q, T p, T &y)
 {
-  using Tol = RmhdTol<T>;
-  if (m_abs(q.PlBx - q.PrBx) > T(Tol::bjump)) return 1;
-  if (isinf(p)) return 1;
-  T Kl[3], Kr[3], Bc[3], etaL, etaR, wL, wR;
-  HlldInner<T> aL, aR;
-  hlld_fill(q, p, Kl, Kr, Bc, etaL, etaR, wL, wR, aL, aR);
-  const T delK = Kr[0] - Kl[0];
-  const T Bch[3] = { Bc[0] * delK, Bc[1] * delK, Bc[2] * delK };
-  const T Yl = (T(1) - dot1(Kl)) / (etaL * delK - dot3(Kl, Bch));
-  const T Yr = (T(1) - dot1(Kr)) / (etaR * delK - dot3(Kr, Bch));
-  if (m_abs(delK) < T(Tol::k_small)) y = T(0);
-  else if (m_abs(Bc[0]) < T(Tol::k_small)) y = delK;
-  else y = delK * (T(1) - Bc[0] * (Yr - Yl));
+  if (isinf(p)) return 1;   // (JumpInNormalBfield cannot occur: one normal field)
+  HlldFill<T> f;
+  hlld_fill(q, p, f);
+  y = hlld_residual(f);
   return 0;
 }
 
@@ -1183,22 +1243,96 @@ __device__ __forceinline__ int hlld_newton(const HlldEqn<T> &q, T &x)
   return 0;
 }
 
-// ReconstructSolution (riemann_hlld-rmhd.cpp:453-575) at s = 0, flux only.
+// The root of equation 48 that hlld_newton finds, with fewer evaluations: one difference slope
+// at the starting pressure, then inverse interpolation through the points already there --
+// Newton's first step and about its second from three evaluations, where the central
+// differences of each Newton iteration take three -- and as in hlld_newton a last step from the
+// point whose residual passes.  Faces on which this does not contract at once (a residual that
+// does not fall, NaN, not below 1e-6 after seven evaluations) run hlld_newton from the start, out of line,
+// so the face keeps the reference's outcome there.  On turbulence faces Newton takes 6 to 12
+// evaluations and this 4 (measured on 240,000 faces; the roots agree to 1e-14 of p).
+struct HlldRoot {
+  double p;
+  int err;
+};
+static __device__ __noinline__ HlldRoot hlld_newton_cold(HlldEqn<double> q, double p)
+{
+  HlldRoot r;
+  r.p = p;
+  r.err = hlld_newton(q, r.p);
+  return r;
+}
+
+// Walks p from the guess to the root of equation 48 (or, with `direct`, stays at it) and leaves
+// the states at the final pressure in f: one evaluation site for the iteration and the flux.
+// `guess` gives the reference's own starting pressure, for hlld_newton.
+template <class Guess>
+__device__ __forceinline__ int hlld_solve(const HlldEqn<double> &q, bool direct, double &p, HlldFill<double> &f,
+                                          const Guess &guess)
+{
+  using Tol = RmhdTol<double>;
+  const double dp = Tol::jac_dp;
+  double x0 = p, y0 = 0.0, s0 = 0.0;     // the start, its residual and dx/dy
+  double x1 = 0.0, y1 = 0.0;             // the latest point
+  bool last = direct;
+#pragma unroll 1
+  for (int it = 0;; ++it) {
+    hlld_fill(q, p, f);
+    if (last) return 0;
+    const double y = hlld_residual(f);
+    if (it == 0) {
+      y0 = y;
+      p = x0 + dp;
+      continue;
+    }
+    bool ok = true;
+    if (it == 1) {
+      s0 = dp / (y - y0);
+      x1 = x0;
+      y1 = y0;
+      p = x0 - s0 * y0;
+    } else {
+      ok = fabs(y) <= 0.02 * fabs(y1) || fabs(y) <= Tol::newton_eps;
+      double step;
+      if (it == 2) {
+        const double t = y0 / (y0 - y);
+        step = s0 * y * t * t;
+      } else {
+        step = y * (p - x1) / (y - y1);
+      }
+      x1 = p;
+      y1 = y;
+      p -= step;
+    }
+    last = fabs(y1) <= Tol::newton_eps;
+    if (!ok || !(fabs(p) < 1e300)) {
+      const HlldRoot r = hlld_newton_cold(q, guess());
+      if (r.err) return 1;
+      p = r.p;
+      last = true;
+    }
+  }
+}
+
+// ReconstructSolution (riemann_hlld-rmhd.cpp:453-575) at s = 0, flux only, from the states f at
+// pressure p.
 template <class T>
-__device__ __forceinline__ int hlld_reconstruct(const HlldEqn<T> &q, T p, T *F)
+__device__ __forceinline__ int hlld_reconstruct(const HlldEqn<T> &q, T p, const HlldFill<T> &f, const Column<T> &col,
+                                                T *F)
 {
   using Tol = RmhdTol<T>;
-  T Kl[3], Kr[3], Bc[3], etaL, etaR, wL, wR;
-  HlldInner<T> aL, aR;
-  hlld_fill(q, p, Kl, Kr, Bc, etaL, etaR, wL, wR, aL, aR);
+  const T (&Kl)[3] = f.Kl, (&Kr)[3] = f.Kr, (&Bc)[3] = f.Bc;
+  const T etaL = f.etaL, etaR = f.etaR, wL = f.wL, wR = f.wR;
+  const HlldInner<T> &aL = f.aL, &aR = f.aR;
   const T am = q.am, ap = q.ap;
   const T denomL = etaL - dot3(Kl, Bc);
   const T denomR = etaR - dot3(Kr, Bc);
   T cLv[3], cRv[3];
+  const Recip<T> iL = recip(denomL), iR = recip(denomR);
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
-    cLv[k] = Kl[k] - Bc[k] * (T(1) - dot1(Kl)) / denomL;
-    cRv[k] = Kr[k] - Bc[k] * (T(1) - dot1(Kr)) / denomR;
+    cLv[k] = Kl[k] - Bc[k] * (T(1) - dot1(Kl)) / iL;
+    cRv[k] = Kr[k] - Bc[k] * (T(1) - dot1(Kr)) / iR;
     if (m_abs(denomL) < T(Tol::k_small)) cLv[k] = aL.v[k];
     if (m_abs(denomR) < T(Tol::k_small)) cRv[k] = aR.v[k];
   }
@@ -1228,11 +1362,13 @@ __device__ __forceinline__ int hlld_reconstruct(const HlldEqn<T> &q, T p, T *F)
   const bool left = region <= 2;
   const HlldJump<T> &J = left ? q.L : q.R;
   const HlldInner<T> &a = left ? aL : aR;
-  const T *Uo = left ? q.Ul : q.Ur;
   const T wave = left ? am : ap;
-  T Fo[8];
+  T Uo[8], Fo[8];
 #pragma unroll
-  for (int i = 0; i < 8; ++i) Fo[i] = left ? q.Fl[i] : q.Fr[i];
+  for (int i = 0; i < 8; ++i) {
+    Uo[i] = col[(left ? 0 : 8) + i];
+    Fo[i] = col[(left ? 16 : 24) + i];
+  }
   if (region == 0 || region == 5) {
 #pragma unroll
     for (int i = 0; i < 8; ++i) F[i] = Fo[i];
@@ -1315,72 +1451,210 @@ __device__ __forceinline__ T hlld_estimate1(T E, T FE, T m, T Fm)
   return (p1 < p2) ? p1 : p2;
 }
 
-// HlldRmhdRiemannSolver::IntercellFlux at s = 0 (riemann_hlld-rmhd.cpp:179-313).
-// Returns 1 when a face state is unphysical (the caller retries with PCM states);
-// `used_hllc` reports the fallback.
-template <class T, int dim>
-__device__ __forceinline__ int riemann_hlld(const PhysParams &pp, const T *pl, const T *pr, T *f, T &ml,
-                                         int &used_hllc, C2PTally *tally)
+// The HLL state's total pressure by the reference's ladder (P: the average face state, its
+// previous state), out of line.
+struct HllState64 {
+  double U[8], P[8];
+};
+struct HllGuess64 {
+  double p;
+  int err, iters, attempts;
+};
+static __device__ __noinline__ HllGuess64 hll_guess64(PhysParams pp, HllState64 s)
 {
-  static_assert(sizeof(T) == sizeof(double), "FP32 faces take riemann_hlld32 (rmhd_face32.cuh)");
+  C2PTally t{0, 0};
+  HllGuess64 o;
+  o.err = cons_to_prim<false, 2>(pp, s.U, s.P, &t);
+  o.iters = t.iters;
+  o.attempts = t.attempts;
+  o.p = hlld_estimate0(s.P);
+  return o;
+}
+
+// An approximate reciprocal, also in the translation units built without fast math.
+__device__ __forceinline__ float rcp32(float x) { return __fdividef(1.f, x); }
+
+// Total pressure of the HLL state, the first pressure guess, by the Anton et al. 2-D Newton in
+// FP32 from (Z, W) of the average face state, to a step of 1e-6 (the guess only seeds the
+// secants, and is kept in FP32): U as D, E, S0..S2, Bx, B1, B2.  Non-zero when the state fails
+// check_cons, Newton does not converge in 32 iterations, or the primitives fail check_prim, with
+// `margin` (of Z for the pressure, of 1 for 1 - v^2) on the last; the caller then takes the FP64
+// ladder.
+__device__ __forceinline__ int hll_pressure32(float gamma, float pfloor, float D, float E, float S0, float S1,
+                                              float S2_, float Bx, float B1, float B2_, float Z, float W, float &pt,
+                                              int &iters, float margin = 0.f)
+{
+  iters = 0;
+  if (!(D >= 0.f) || !(E - D >= 0.f)) return 1;
+  const float gamf = (gamma - 1.f) / gamma;
+  const float S2 = S0 * S0 + S1 * S1 + S2_ * S2_;
+  const float B2 = Bx * Bx + B1 * B1 + B2_ * B2_;
+  const float BS = Bx * S0 + B1 * S1 + B2_ * S2_;
+  const float BS2 = BS * BS;
+  const float iD = rcp32(D);
+  float iW = rcp32(W), iZ = rcp32(Z);
+#pragma unroll 1
+  for (;;) {
+    const float W2 = W * W, iW2 = iW * iW, iW3 = iW2 * iW, iZ2 = iZ * iZ, iZ3 = iZ2 * iZ;
+    const float T = BS2 * iZ2;
+    const float BZ = B2 + Z, u2 = (W2 - 1.f) * iW2;
+    const float Pre = (Z * iW2 - D * iW) * gamf;
+    const float f0Z = 2.f * BZ * (BS2 * iZ3 + u2);
+    const float f0W = 2.f * BZ * BZ * iW3;
+    const float f1Z = 1.f + BS2 * iZ3 - gamf * iW2;
+    const float f1W = (B2 + (2.f * Z - D * W) * gamf) * iW3;
+    const float f0 = BZ * BZ * u2 - (2.f * Z + B2) * T - S2;
+    const float f1 = Z + B2 - E - Pre - 0.5f * B2 * iW2 - 0.5f * T;
+    const float idet = rcp32(f0Z * f1W - f0W * f1Z);
+    const float dZ = -(f1W * f0 - f0W * f1) * idet;
+    const float dW = -(f0Z * f1 - f1Z * f0) * idet;
+    const float Zn = fabsf(Z + dZ);
+    Z = (Zn < 1e20f) ? Zn : Z;
+    W = fminf(fmaxf(W + dW, 1.f), 1e12f);
+    iZ = rcp32(Z);
+    iW = rcp32(W);
+    const float err = fabsf(dZ * iZ) + fabsf(dW * iW);
+    ++iters;
+    if (!(err > 1e-6f)) {
+      if (!(err == err)) return 1;
+      break;
+    }
+    if (iters == 32) return 1;
+  }
+  const float r = D * iW;
+  float p = r * (Z * iD * iW - 1.f) * gamf;
+  if (pfloor > 0.f && p < pfloor) p = pfloor;
+  const float vB = BS * iZ, iZB = rcp32(Z + B2);
+  const float v2 = (S2 + vB * (2.f * BS + vB * B2)) * iZB * iZB;
+  if (!(v2 < 1.f - margin) || !(p >= margin * Z) || !(r >= 0.f)) return 1;
+  pt = p + 0.5f * (B2 * (1.f - v2) + vB * vB);
+  return 0;
+}
+
+// HlldRmhdRiemannSolver::IntercellFlux at s = 0 (riemann_hlld-rmhd.cpp:179-313), FP64 (FP32 faces
+// take riemann_hlld32, rmhd_face32.cuh).  The face's states come in the first 16 entries of
+// this thread's column -- left, then right, in the normal frame of dim -- and the column then
+// holds both sides' U (0..15) and F (16..31): they are needed again only for the
+// outermost flux, and in registers they would halve the resident warps.  One copy of the side's
+// code serves both sides, and one of the inner states' code serves the pressure iteration and
+// the flux: with every copy inlined the kernel was 520 KB, and up to a third of its warps'
+// waiting was for instructions.
+// Returns 1 when a face state is unphysical (the caller retries with PCM states); `used_hllc`
+// reports the fallback; `src` gives the two face states again, in the reference's component
+// order, on the rare paths.  The flux f is in the normal frame.
+template <class Src>
+__device__ __forceinline__ int riemann_hlld64(const PhysParams &pp, int dim, const Column<double> &col, double *f,
+                                              double &ml, int &used_hllc, C2PTally *tally, const Src &src)
+{
+  using T = double;
   using Tol = RmhdTol<T>;
   const T gamma = T(pp.gamma);
-  using M = DimMap<dim>;
-  constexpr int B1 = M::B1, B2 = M::B2, B3 = M::B3, S1 = M::S1, S2 = M::S2, S3 = M::S3;
-  constexpr int v1 = M::v1, v2 = M::v2, v3 = M::v3;
   HlldEqn<T> q;
-  T Pl[8], Pr[8], epl, eml, epr, emr;
-  Pl[pre] = pl[pre]; Pr[pre] = pr[pre];
-  Pl[rho] = pl[rho]; Pr[rho] = pr[rho];
-  Pl[vx] = pl[v1];   Pr[vx] = pr[v1];
-  Pl[vy] = pl[v2];   Pr[vy] = pr[v2];
-  Pl[vz] = pl[v3];   Pr[vz] = pr[v3];
-  Pl[By] = pl[B2];   Pr[By] = pr[B2];
-  Pl[Bz] = pl[B3];   Pr[Bz] = pr[B3];
-  Pl[Bx] = Pr[Bx] = T(0.5) * (pl[B1] + pr[B1]);
+  q.bx = T(0.5) * (col[Bx] + col[8 + Bx]);
   used_hllc = 0;
   if (tally) { tally->iters = 0; tally->attempts = 0; }
-  if (prim_to_cons(gamma, Pl, q.Ul)) return 1;
-  if (prim_to_cons(gamma, Pr, q.Ur)) return 1;
-  flux_and_eigenvalues(gamma, q.Ul, Pl, q.Fl, epl, eml, 1);
-  flux_and_eigenvalues(gamma, q.Ur, Pr, q.Fr, epr, emr, 1);
-  const T am = (eml < emr) ? eml : emr;
-  const T ap = (epl > epr) ? epl : epr;
+  T ap = T(0), am = T(0);
+  float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f, a4 = 0.f;   // the average face state: rho, p, v
+#pragma unroll 1
+  for (int side = 0; side < 2; ++side) {
+    const Column<T> u{col.p + 8 * side * col.stride, col.stride}, w{col.p + (16 + 8 * side) * col.stride, col.stride};
+    T P[8], U[8], F[8], ep, em;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) P[i] = u[i];
+    P[Bx] = q.bx;
+    a0 += 0.5f * float(P[rho]);
+    a1 += 0.5f * float(P[pre]);
+    a2 += 0.5f * float(P[vx]);
+    a3 += 0.5f * float(P[vy]);
+    a4 += 0.5f * float(P[vz]);
+    if (prim_to_cons(gamma, P, U)) return 1;
+    flux_and_eigenvalues(gamma, U, P, F, ep, em, 1);
+    am = (side == 0 || em < am) ? em : am;
+    ap = (side == 0 || ep > ap) ? ep : ap;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      u[i] = U[i];
+      w[i] = F[i];
+    }
+  }
   const T l = face_lambda(ap, am);
   if (ml < l) ml = l;
-  T P_hll[8], U_hll[8], F_hll[8];
+  // The HLL state and flux, and from them the first pressure guess.  The iteration converges to
+  // the same root from a guess good to 1e-6, so the HLL state is inverted in FP32 where its
+  // pressure and velocity are clear of the checks the reference's inversion makes; elsewhere,
+  // and for the faces that run the reference's own Newton, in FP64 (hll_guess64).
+  T U_hll[8], F_hll[3];
+  {
+    const Recip<T> iS = recip(ap - am);
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    P_hll[i] = T(0.5) * (Pl[i] + Pr[i]);
-    U_hll[i] = (ap * q.Ur[i] - am * q.Ul[i] + (q.Fl[i] - q.Fr[i])) / (ap - am);
-    F_hll[i] = (ap * q.Fl[i] - am * q.Fr[i] + ap * am * (q.Ur[i] - q.Ul[i])) / (ap - am);
+    for (int i = 0; i < 8; ++i) {
+      const T ul = col[i], ur = col[8 + i], fl = col[16 + i], fr = col[24 + i];
+      U_hll[i] = (ap * ur - am * ul + (fl - fr)) / iS;
+      if (i < 3) F_hll[i] = (ap * fl - am * fr + ap * am * (ur - ul)) / iS;
+    }
   }
-  const int hll_c2p_failed = cons_to_prim<false, 2>(pp, U_hll, P_hll, tally);
+  const auto guess64 = [&](double &p) {
+    double ql[8], qr[8];
+    src(ql, qr);
+    HllState64 h;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      h.U[i] = U_hll[i];
+      h.P[i] = T(0.5) * (ql[frame_slot(dim, i)] + qr[frame_slot(dim, i)]);
+    }
+    h.P[Bx] = q.bx;
+    const HllGuess64 o = hll_guess64(pp, h);
+    p = o.p;
+    if (tally) { tally->iters = o.iters; tally->attempts = o.attempts; }
+    return o.err;
+  };
+  const bool direct = m_abs(q.bx) < T(Tol::bx_small);
+  T p_est0;
+  int hll_c2p_failed;
+  {
+    const float g = float(gamma), i2 = 1.f - (a2 * a2 + a3 * a3 + a4 * a4);
+    const float W2 = rcp32(i2);
+    float pt = 0.f;
+    int it = 0;
+    hll_c2p_failed = !(i2 > 0.f && a0 > 0.f && a1 > 0.f) ||
+                     hll_pressure32(g, float(pp.pfloor), float(U_hll[ddd]), float(U_hll[tau] + U_hll[ddd]),
+                                    float(U_hll[Sx]), float(U_hll[Sy]), float(U_hll[Sz]), float(U_hll[Bx]),
+                                    float(U_hll[By]), float(U_hll[Bz]), (a0 + g * rcp32(g - 1.f) * a1) * W2,
+                                    sqrtf(W2), pt, it, 1e-3f);
+    p_est0 = T(pt);
+    if (tally) { tally->iters = it; tally->attempts = 1; }
+    if (hll_c2p_failed) hll_c2p_failed = guess64(p_est0);
+  }
   // HlldEquation48 constructor (riemann_hlld-rmhd.cpp:315-345)
-  q.ap = ap; q.am = am; q.PlBx = Pl[Bx]; q.PrBx = Pr[Bx];
-  q.Ul[tau] += q.Ul[ddd];
-  q.Fl[tau] += q.Fl[ddd];
-  q.Ur[tau] += q.Ur[ddd];
-  q.Fr[tau] += q.Fr[ddd];
-  q.L.E = am * q.Ul[tau] - q.Fl[tau];
-  q.R.E = ap * q.Ur[tau] - q.Fr[tau];
-  q.L.D = am * q.Ul[ddd] - q.Fl[ddd];
-  q.R.D = ap * q.Ur[ddd] - q.Fr[ddd];
+  q.ap = ap;
+  q.am = am;
+  {
+    const T El = col[tau] + col[ddd], FEl = col[16 + tau] + col[16 + ddd];
+    const T Er = col[8 + tau] + col[8 + ddd], FEr = col[24 + tau] + col[24 + ddd];
+    col[tau] = El;
+    col[16 + tau] = FEl;
+    col[8 + tau] = Er;
+    col[24 + tau] = FEr;
+    q.L.E = am * El - FEl;
+    q.R.E = ap * Er - FEr;
+    q.L.D = am * col[ddd] - col[16 + ddd];
+    q.R.D = ap * col[8 + ddd] - col[24 + ddd];
+  }
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
-    q.L.B[k] = am * q.Ul[Bx + k] - q.Fl[Bx + k];
-    q.R.B[k] = ap * q.Ur[Bx + k] - q.Fr[Bx + k];
-    q.L.m[k] = am * q.Ul[Sx + k] - q.Fl[Sx + k];
-    q.R.m[k] = ap * q.Ur[Sx + k] - q.Fr[Sx + k];
+    q.L.B[k] = am * col[Bx + k] - col[16 + Bx + k];
+    q.R.B[k] = ap * col[8 + Bx + k] - col[24 + Bx + k];
+    q.L.m[k] = am * col[Sx + k] - col[16 + Sx + k];
+    q.R.m[k] = ap * col[8 + Sx + k] - col[24 + Sx + k];
   }
   T F[8];
   int attempt = 0, success = 0;
+#pragma unroll 1
   while (!hll_c2p_failed && attempt < 3 && !success) {
     T p_star;
-    int rc;
-    const int est = (m_abs(Pl[Bx]) < T(Tol::bx_small) || m_abs(Pr[Bx]) < T(Tol::bx_small)) ? 1 : attempt;
+    const int est = direct ? 1 : attempt;
     if (est == 0) {
-      p_star = hlld_estimate0(P_hll);
+      p_star = p_est0;
     } else if (est == 1) {   // EstimateSolution(1) shifts tau and restores it afterwards
       F_hll[tau] += F_hll[ddd];
       U_hll[tau] += U_hll[ddd];
@@ -1390,31 +1664,27 @@ __device__ __forceinline__ int riemann_hlld(const PhysParams &pp, const T *pl, c
     } else {
       p_star = T(0);
     }
-    if (m_abs(Pl[Bx]) < T(Tol::bx_small) || m_abs(Pr[Bx]) < T(Tol::bx_small)) {
-      rc = hlld_reconstruct(q, p_star, F);
-    } else {
-      rc = hlld_newton(q, p_star);
-      if (rc == 0) rc = hlld_reconstruct(q, p_star, F);
-    }
+    const T p_star0 = p_star;
+    HlldFill<T> fill;
+    const auto start = [&]() {
+      double p = p_star0;
+      if (est == 0) guess64(p);
+      return p;
+    };
+    int rc = hlld_solve(q, direct, p_star, fill, start);
+    if (rc == 0) rc = hlld_reconstruct(q, p_star, fill, col, F);
     success = (rc == 0);
     ++attempt;
   }
   if (success) {
-    f[ddd] = F[ddd];
-    f[tau] = F[tau];
-    f[S1] = F[Sx];
-    f[S2] = F[Sy];
-    f[S3] = F[Sz];
-    f[B1] = F[Bx];
-    f[B2] = F[By];
-    f[B3] = F[Bz];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) f[i] = F[i];
     return 0;
   }
   used_hllc = 1;
   Face8<T> a, b;
-#pragma unroll
-  for (int i = 0; i < 8; ++i) { a.v[i] = pl[i]; b.v[i] = pr[i]; }
-  const HllcOut<T> o = riemann_hllc_fallback<T, dim>(gamma, a, b, ml);
+  src(a.v, b.v);
+  const HllcOut<T> o = riemann_hllc_fallback<T>(dim, gamma, a, b, ml);
   ml = o.ml;
 #pragma unroll
   for (int i = 0; i < 8; ++i) f[i] = o.F[i];

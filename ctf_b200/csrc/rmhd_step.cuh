@@ -339,108 +339,188 @@ struct FluxTally {
   int hlld_ok, hlld_hllc, pcm_retry, face_c2p_calls, face_c2p_iters;
 };
 
-// The two states of the face between zones f and f + S: reconstructed, or with retry the zone
-// states themselves.  The reconstruction is chosen once, outside the component loops, so that
-// each loop's loads are issued together.
+// The component that slot q of a face's states and flux holds: the HLLD solvers and the FP32 HLLC
+// work in the normal frame of the sweep direction, HLL and the FP64 HLLC in the reference's
+// component order.
+template <class T, int RS> __host__ __device__ constexpr int face_slot(int dim, int q)
+{
+  return RS == RIEMANN_HLLD || (RS == RIEMANN_HLLC && sizeof(T) < sizeof(double)) ? frame_slot(dim, q) : q;
+}
+
+// The slot that component c goes to: face_slot's inverse.
+template <class T, int RS> __host__ __device__ constexpr int slot_of(int dim, int c)
+{
+  if (face_slot<T, RS>(2, 2) == 2) return c;
+  return c < 2 ? c : c < 5 ? 2 + (c - 2 + 4 - dim) % 3 : 5 + (c - 5 + 4 - dim) % 3;
+}
+
+// The two states of one component of the face between zones a and a + S: reconstructed by
+// `recon`.
 template <class T>
-__device__ __forceinline__ void face_states(const T *__restrict__ PA, long long cs, long long S, const PhysParams &pp,
+__device__ __forceinline__ void face_component(const T *__restrict__ a, long long S, const PhysParams &pp, int recon,
+                                               T theta, T &l, T &r)
+{
+  if (recon == RECON_PCM) {
+    l = a[0];
+    r = a[S];
+  } else if (recon == RECON_PLM) {
+    const T vm = a[-S], v0 = a[0], vp = a[S], vpp = a[2 * S];
+    l = plm(theta, vm, v0, vp, T(+1));
+    r = plm(theta, v0, vp, vpp, T(-1));
+  } else {
+    const T vm2 = a[-2 * S], vm1 = a[-S], v0 = a[0], vp1 = a[S], vp2 = a[2 * S], vp3 = a[3 * S];
+    l = weno5(pp.is_mode, T(pp.sz10A), vm2, vm1, v0, vp1, vp2, true);
+    r = weno5(pp.is_mode, T(pp.sz10A), vm1, v0, vp1, vp2, vp3, false);
+  }
+}
+
+// The two states of the face between zones f and f + S of direction dim: reconstructed, or with
+// retry the zone states themselves.  The reconstruction is chosen once, outside the component
+// loops, so that each loop's loads are issued together.
+template <class T, int RS>
+__device__ __forceinline__ void face_states(const Grid &g, const T *__restrict__ PA, const PhysParams &pp, int dim,
                                             long long f, bool retry, T *Pl, T *Pr)
 {
-  const T *a = PA + f;
-  if (retry || pp.recon == RECON_PCM) {
-#pragma unroll
-    for (int q = 0; q < 8; ++q, a += cs) {
-      Pl[q] = a[0];
-      Pr[q] = a[S];
-    }
-  } else if (pp.recon == RECON_PLM) {
-    const T theta = T(pp.theta);
-#pragma unroll
-    for (int q = 0; q < 8; ++q, a += cs) {
-      const T vm = a[-S], v0 = a[0], vp = a[S], vpp = a[2 * S];
-      Pl[q] = plm(theta, vm, v0, vp, T(+1));
-      Pr[q] = plm(theta, v0, vp, vpp, T(-1));
-    }
-  } else {
-#pragma unroll
-    for (int q = 0; q < 8; ++q, a += cs) {
-      const T vm2 = a[-2 * S], vm1 = a[-S], v0 = a[0], vp1 = a[S], vp2 = a[2 * S], vp3 = a[3 * S];
-      Pl[q] = weno5(pp.is_mode, T(pp.sz10A), vm2, vm1, v0, vp1, vp2, true);
-      Pr[q] = weno5(pp.is_mode, T(pp.sz10A), vm1, v0, vp1, vp2, vp3, false);
-    }
-  }
+  const long long S = g.s[dim - 1];
+  const T theta = T(pp.theta);
+#define MGPU_FACE_LOOP(R)                                                                                   \
+  _Pragma("unroll") for (int q = 0; q < 8; ++q)                                                             \
+      face_component<T>(PA + face_slot<T, RS>(dim, q) * g.cs + f, S, pp, R, theta, Pl[q], Pr[q])
+  if (retry || pp.recon == RECON_PCM) { MGPU_FACE_LOOP(RECON_PCM); }
+  else if (pp.recon == RECON_PLM) { MGPU_FACE_LOOP(RECON_PLM); }
+  else { MGPU_FACE_LOOP(RECON_WENO5); }
+#undef MGPU_FACE_LOOP
 }
 
-// Both face values of zone z along stride S: lo toward z - S, hi toward z + S, which are
+// The same into this thread's column (left 0..7, right 8..15), one component at a time: an eighth
+// of the code of the unrolled form, which in FP64 is long (WENO5 divides eight times per
+// component).
+template <class T, int RS>
+__device__ __forceinline__ void face_states_column(const Grid &g, const T *__restrict__ PA, const PhysParams &pp,
+                                                   int dim, long long f, bool retry, const Column<T> &col)
+{
+  const long long S = g.s[dim - 1];
+  const T theta = T(pp.theta);
+  const int recon = retry ? (int) RECON_PCM : pp.recon;
+#pragma unroll 1
+  for (int q = 0; q < 8; ++q)
+    face_component<T>(PA + face_slot<T, RS>(dim, q) * g.cs + f, S, pp, recon, theta, col[q], col[8 + q]);
+}
+
+// Both face values of zone z along direction dim: lo toward z - S, hi toward z + S, which are
 // face_states' Pr of the face below and Pl of the face above.
-template <class T>
-__device__ __forceinline__ void zone_states(const T *__restrict__ PA, long long cs, long long S, const PhysParams &pp,
+template <class T, int RS>
+__device__ __forceinline__ void zone_states(const Grid &g, const T *__restrict__ PA, const PhysParams &pp, int dim,
                                             long long z, T *lo, T *hi)
 {
+  const long long S = g.s[dim - 1];
   const T *a = PA + z;
+  // components in memory order, each into its slot of the normal frame
+#define MGPU_ZONE_LOOP(expr)                             \
+  _Pragma("unroll") for (int c = 0; c < 8; ++c, a += g.cs) { \
+    const int q = slot_of<T, RS>(dim, c);                \
+    expr;                                                \
+  }
   if (pp.recon == RECON_PCM) {
-#pragma unroll
-    for (int q = 0; q < 8; ++q, a += cs) lo[q] = hi[q] = a[0];
+    MGPU_ZONE_LOOP(lo[q] = hi[q] = a[0])
   } else if (pp.recon == RECON_PLM) {
     const T theta = T(pp.theta);
-#pragma unroll
-    for (int q = 0; q < 8; ++q, a += cs) plm_zone(theta, a[-S], a[0], a[S], lo[q], hi[q]);
+    MGPU_ZONE_LOOP(plm_zone(theta, a[-S], a[0], a[S], lo[q], hi[q]))
   } else {
-#pragma unroll
-    for (int q = 0; q < 8; ++q, a += cs)
-      weno5_zone(pp.is_mode, T(pp.sz10A), a[-2 * S], a[-S], a[0], a[S], a[2 * S], lo[q], hi[q]);
+    MGPU_ZONE_LOOP(weno5_zone(pp.is_mode, T(pp.sz10A), a[-2 * S], a[-S], a[0], a[S], a[2 * S], lo[q], hi[q]))
   }
+#undef MGPU_ZONE_LOOP
 }
 
-// A face's states fetched again on the rare paths of the FP32 HLLD solver (out of line).
-struct FaceStates32 {
-  float l[8], r[8];
+// A face's states (reference component order) fetched again on the rare paths of the HLLD
+// solvers, out of line.
+template <class T> struct FaceStates {
+  T l[8], r[8];
 };
-static __device__ __noinline__ FaceStates32 refetch_face(const float *PA, long long cs, long long S, PhysParams pp,
-                                                         long long f, bool retry)
+template <class T>
+static __device__ __noinline__ FaceStates<T> refetch_face(const T *PA, long long cs, long long S, PhysParams pp,
+                                                          long long f, bool retry)
 {
-  FaceStates32 o;
-  face_states<float>(PA, cs, S, pp, f, retry, o.l, o.r);
+  FaceStates<T> o;
+  const int recon = retry ? (int) RECON_PCM : pp.recon;
+#pragma unroll 1
+  for (int q = 0; q < 8; ++q) face_component<T>(PA + q * cs + f, S, pp, recon, T(pp.theta), o.l[q], o.r[q]);
   return o;
 }
 
-// The flux of the face between zones f and f + S from its states Pl, Pr (overwritten by the PCM
-// retry), in Fo (zero when both attempts fail); the face's |lambda| is folded into ml.
-template <class T, int dim, int RS>
-__device__ __forceinline__ void solve_face(const Grid &g, const T *__restrict__ PA, const PhysParams &pp, long long f,
-                                           T *Pl, T *Pr, T &ml, FluxTally &ft, T *Fo)
+// Whether a sweep of Riemann solver RS keeps its states in columns of shared memory
+// (riemann_hlld64), and the entries per thread.
+template <class T, int RS> __host__ __device__ constexpr bool uses_column()
+{
+  return RS == RIEMANN_HLLD && sizeof(T) == sizeof(double);
+}
+template <class T, int RS> __host__ __device__ constexpr int column_entries() { return uses_column<T, RS>() ? 32 : 1; }
+
+// The Riemann solver at one face of direction dim.
+template <class T, int RS, class Src>
+__device__ __forceinline__ int riemann_face(const PhysParams &pp, int dim, const T *Pl, const T *Pr, T *Fo, T &ml,
+                                            int &used_hllc, C2PTally *t, const Column<T> &col, const Src &src)
+{
+  const T gamma = T(pp.gamma);
+  if constexpr (RS == RIEMANN_HLLD) {
+    if constexpr (sizeof(T) < sizeof(double)) return riemann_hlld32(pp, dim, Pl, Pr, Fo, ml, used_hllc, t, src);
+    else return riemann_hlld64(pp, dim, col, Fo, ml, used_hllc, t, src);
+  } else if constexpr (RS == RIEMANN_HLLC && sizeof(T) < sizeof(double)) {
+    return riemann_hllc32(gamma, Pl, Pr, Fo, ml);
+  } else if constexpr (RS == RIEMANN_HLLC) {
+    if (dim == 1) return riemann_hllc<T, 1>(gamma, Pl, Pr, Fo, ml);
+    if (dim == 2) return riemann_hllc<T, 2>(gamma, Pl, Pr, Fo, ml);
+    return riemann_hllc<T, 3>(gamma, Pl, Pr, Fo, ml);
+  } else {
+    if (dim == 1) return riemann_hll<T, 1>(gamma, Pl, Pr, Fo, ml);
+    if (dim == 2) return riemann_hll<T, 2>(gamma, Pl, Pr, Fo, ml);
+    return riemann_hll<T, 3>(gamma, Pl, Pr, Fo, ml);
+  }
+}
+
+// The flux of the face between zones f and f + S of direction dim, in Fo (face_slot's order; zero
+// when both attempts fail); the face's |lambda| is folded into ml.  `given`: its states are in
+// Pl, Pr (the marching sweeps); otherwise they are reconstructed here.  Attempt 1 takes the
+// zone states themselves (the PCM retry).  colp: this thread's column (uses_column), 128 apart.
+template <class T, int RS, bool given>
+__device__ __forceinline__ void solve_face(const Grid &g, const T *__restrict__ PA, const PhysParams &pp, int dim,
+                                           long long f, T *Pl, T *Pr, T &ml, FluxTally &ft, T *Fo, T *colp)
 {
   const long long S = g.s[dim - 1];
-  const T gamma = T(pp.gamma);
   int err = 1, used_hllc = 0;
-  constexpr bool hlld = RS == RIEMANN_HLLD;
   C2PTally tally{0, 0};
-  // attempt 0: reconstructed states; attempt 1: the zone states themselves (PCM retry).
+  const Column<T> col{colp, 128};
+  if constexpr (!given && !uses_column<T, RS>()) face_states<T, RS>(g, PA, pp, dim, f, false, Pl, Pr);
+  if constexpr (given && uses_column<T, RS>()) {
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      col[q] = Pl[q];
+      col[8 + q] = Pr[q];
+    }
+  }
   // One call site per solver keeps a single inlined copy of it.
 #pragma unroll 1
   for (int attempt = 0; attempt < 2 && err; ++attempt) {
-    if (attempt == 1) {
-      ft.pcm_retry += 1;
+    if (attempt == 1) ft.pcm_retry += 1;
+    if constexpr (uses_column<T, RS>()) {
+      if (!given || attempt == 1) face_states_column<T, RS>(g, PA, pp, dim, f, attempt == 1, col);
+    } else if (attempt == 1) {
 #pragma unroll
       for (int q = 0; q < 8; ++q) {
-        Pl[q] = PA[q * g.cs + f];
-        Pr[q] = PA[q * g.cs + f + S];
+        Pl[q] = PA[face_slot<T, RS>(dim, q) * g.cs + f];
+        Pr[q] = PA[face_slot<T, RS>(dim, q) * g.cs + f + S];
       }
     }
     C2PTally t{0, 0};
-    if constexpr (RS == RIEMANN_HLLD && sizeof(T) < sizeof(double)) {
-      const auto src = [&](float *l, float *r) {
-        const FaceStates32 o = refetch_face(PA, g.cs, S, pp, f, attempt == 1);
+    const auto src = [&](T *l, T *r) {
+      const FaceStates<T> o = refetch_face<T>(PA, g.cs, S, pp, f, attempt == 1);
 #pragma unroll
-        for (int q = 0; q < 8; ++q) {
-          l[q] = o.l[q];
-          r[q] = o.r[q];
-        }
-      };
-      err = riemann_hlld32<dim>(pp, Pl, Pr, Fo, ml, used_hllc, &t, src);
-    } else if constexpr (RS == RIEMANN_HLLD) err = riemann_hlld<T, dim>(pp, Pl, Pr, Fo, ml, used_hllc, &t);
-    else if constexpr (RS == RIEMANN_HLLC) err = riemann_hllc<T, dim>(gamma, Pl, Pr, Fo, ml);
-    else err = riemann_hll<T, dim>(gamma, Pl, Pr, Fo, ml);
+      for (int q = 0; q < 8; ++q) {
+        l[q] = o.l[q];
+        r[q] = o.r[q];
+      }
+    };
+    err = riemann_face<T, RS>(pp, dim, Pl, Pr, Fo, ml, used_hllc, &t, col, src);
     tally.iters += t.iters;
     tally.attempts += t.attempts;
   }
@@ -448,7 +528,7 @@ __device__ __forceinline__ void solve_face(const Grid &g, const T *__restrict__ 
 #pragma unroll
     for (int q = 0; q < 8; ++q) Fo[q] = T(0);
   }
-  if constexpr (hlld) {
+  if constexpr (RS == RIEMANN_HLLD) {
     ft.hlld_ok += 1 - used_hllc;
     ft.hlld_hllc += used_hllc;
   }
@@ -456,25 +536,15 @@ __device__ __forceinline__ void solve_face(const Grid &g, const T *__restrict__ 
   ft.face_c2p_iters += tally.iters;
 }
 
-// One face: reconstruct and solve.
-template <class T, int dim, int RS>
-__device__ __forceinline__ void face_flux(const Grid &g, const T *__restrict__ PA, const PhysParams &pp, long long f,
-                                          T &ml, FluxTally &ft, T *Fo)
-{
-  T Pl[8], Pr[8];
-  face_states<T>(PA, g.cs, g.s[dim - 1], pp, f, false, Pl, Pr);
-  solve_face<T, dim, RS>(g, PA, pp, f, Pl, Pr, ml, ft, Fo);
-}
-
 // One face, its flux stored in F.
-template <class T, int dim, int RS>
+template <class T, int RS>
 __device__ __forceinline__ void flux_face(const Grid &g, const T *__restrict__ PA, T *__restrict__ F,
-                                          const PhysParams &pp, long long f, T &ml, FluxTally &ft)
+                                          const PhysParams &pp, int dim, long long f, T &ml, FluxTally &ft, T *colp)
 {
-  T Fo[8];
-  face_flux<T, dim, RS>(g, PA, pp, f, ml, ft, Fo);
+  T Pl[8], Pr[8], Fo[8];
+  solve_face<T, RS, false>(g, PA, pp, dim, f, Pl, Pr, ml, ft, Fo, colp);
 #pragma unroll
-  for (int q = 0; q < 8; ++q) F[q * g.cs + f] = Fo[q];
+  for (int q = 0; q < 8; ++q) F[face_slot<T, RS>(dim, q) * g.cs + f] = Fo[q];
 }
 
 // MaxLambda of a block: warp max -> block max -> one atomicMax (non-negative doubles order
@@ -504,16 +574,26 @@ __device__ __forceinline__ void flux_block_finish(double m, const FluxTally &ft,
   warp_add(&st.face_c2p_iters, (unsigned) ft.face_c2p_iters);
 }
 
-template <class T, int dim, int RS>
-__global__ void __launch_bounds__(128, flux_minb<RS>()) k_flux(Grid g, const T *__restrict__ PA, T *__restrict__ F,
-                                                              PhysParams pp, Ctl *ctl, int stage)
+// The faces of every direction in one launch: blocks [0, n1) sweep x, [n1, n2) y, the rest z.  The
+// sweeps are independent, a face's latency is some ten microseconds in FP32 and over fifty in
+// FP64, and a small box fills less than one wave of blocks per direction, so one launch takes
+// little more than one sweep where three took three: 16^3 FP64 flux 0.62 -> 0.24 ms per RK2
+// step.  Large boxes gain the tails of two launches.
+template <class T, int RS>
+__global__ void __launch_bounds__(128, flux_minb<RS>()) k_flux(Grid g, const T *__restrict__ PA, T *__restrict__ F0,
+                                                              T *__restrict__ F1, T *__restrict__ F2, unsigned n1,
+                                                              unsigned n2, PhysParams pp, Ctl *ctl, int stage)
 {
   if (stage_failed(ctl, stage + 1)) return;
+  const int dim = blockIdx.x < n1 ? 1 : blockIdx.x < n2 ? 2 : 3;
+  const unsigned b = blockIdx.x - (dim == 1 ? 0u : dim == 2 ? n1 : n2);
+  T *F = dim == 1 ? F0 : dim == 2 ? F1 : F2;
   const long long S = g.s[dim - 1];
-  const long long f = 2 * S + (long long) blockIdx.x * blockDim.x + threadIdx.x;
+  const long long f = 2 * S + (long long) b * blockDim.x + threadIdx.x;
   T ml = T(0);
   FluxTally ft{0, 0, 0, 0, 0};
-  if (f < g.nz - 3 * S) flux_face<T, dim, RS>(g, PA, F, pp, f, ml, ft);
+  __shared__ T cols[column_entries<T, RS>() * 128];
+  if (f < g.nz - 3 * S) flux_face<T, RS>(g, PA, F, pp, dim, f, ml, ft, cols + threadIdx.x);
   flux_block_finish(double(ml), ft, ctl, RS == RIEMANN_HLLD);
 }
 
