@@ -32,7 +32,7 @@ class HostCopyPool {
   // returns when every part is copied.  Not reentrant: one copy at a time.
   void copy(void *dst, const void *src, size_t bytes)
   {
-    if (n_ == 1 || bytes < (size_t(8) << 20)) {
+    if (n_ == 1 || bytes < (size_t(1) << 20)) {   // a wake-up costs what a thread copies in that time
       memcpy(dst, src, bytes);
       return;
     }

@@ -6,6 +6,7 @@
 #include <stdint.h>
 #include <stdio.h>
 #include <string.h>
+#include <algorithm>
 #include <chrono>
 #include <string>
 #include <vector>
@@ -452,14 +453,23 @@ int mgpu_num_zones(const mgpu_solver *h, long long *nz)
 
 static bool pipe_host_setup(mgpu_solver *h);
 
-// Two pinned slots of the device staging chunk's size and two events, for the chunked host
-// transfers of a large pageable buffer, and the copy threads; false when they cannot be had
-// (the copies then read and write the pageable buffer directly).
+// Zones of a chunk of a staged host transfer of `zones` zones, so that the host copy of one chunk
+// overlaps the DMA copy of the previous one: 2 MB up to 64 MB (pinning the two slots costs a
+// solver's first transfer about 2 ms per MB), then a quarter of the array up to 64 MB.
+static long long xfer_chunk(const mgpu_solver *h, long long zones)
+{
+  const long long most = std::min<long long>(h->staging_zones, 1ll << 20);
+  return std::min(most, zones <= (1ll << 20) ? 1ll << 15 : (zones + 3) / 4);
+}
+
+// Two pinned slots of a whole-array transfer's chunk and two events, for the chunked host
+// transfers of a pageable buffer, and the copy threads; false when they cannot be had (the
+// copies then read and write the pageable buffer directly).
 static bool xfer_host_setup(mgpu_solver *h)
 {
   if (h->xfer_host_state == 0) {
-    cudaError_t e = cudaHostAlloc((void **) &h->xfer_host, (size_t) h->staging_zones * 2 * 8 * sizeof(double),
-                                  cudaHostAllocDefault);
+    cudaError_t e = cudaHostAlloc((void **) &h->xfer_host,
+                                  (size_t) xfer_chunk(h, h->g.nz) * 2 * 8 * sizeof(double), cudaHostAllocDefault);
     while (h->xfer_ev.size() < 2 && e == cudaSuccess) {   // the events outlive a new domain
       cudaEvent_t ev;
       e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
@@ -510,20 +520,22 @@ static int transfer(mgpu_solver *h, double *host, const void *dev_in, void *dev_
     CK(cudaStreamSynchronize(h->stream));
     return MGPU_OK;
   }
-  // a large pageable buffer goes through two pinned chunk slots (xfer_host), chunk by chunk:
-  // the threaded host copy of one chunk overlaps the DMA copy and conversion of the other
+  // a pageable buffer from 4 MB on goes through two pinned chunk slots (xfer_host), chunk by chunk:
+  // the threaded host copy of one chunk overlaps the DMA copy and conversion of the other (the
+  // driver moves pageable memory at about 13 GB/s; a 64^3 FP64 Mara.advance, 22 MB each way,
+  // took 4.8 ms with the driver's copies)
   bool staged = false;
-  if ((size_t) (nz - zbeg) * 8 * sizeof(double) >= (size_t(64) << 20)) {
+  if ((size_t) (nz - zbeg) * 8 * sizeof(double) >= (size_t(4) << 20)) {
     cudaPointerAttributes pa{};
     const bool pinned = cudaPointerGetAttributes(&pa, host + zbeg * 8) == cudaSuccess && pa.type == cudaMemoryTypeHost;
     cudaGetLastError();   // an unregistered pointer may leave an error behind
     staged = !pinned && xfer_host_setup(h);
   }
-  const long long slot_doubles = h->staging_zones * 8;
+  const long long chunk = staged ? xfer_chunk(h, nz - zbeg) : h->staging_zones, slot_doubles = chunk * 8;
   auto slot = [&](int c) { return h->xfer_host + (c % 2) * slot_doubles; };
   int nchunk = 0;
-  for (long long z0 = zbeg; z0 < nz; z0 += h->staging_zones) {
-    const long long cnt = (nz - z0) < h->staging_zones ? (nz - z0) : h->staging_zones;
+  for (long long z0 = zbeg; z0 < nz; z0 += chunk) {
+    const long long cnt = (nz - z0) < chunk ? (nz - z0) : chunk;
     const size_t bytes = (size_t) cnt * 8 * sizeof(double);
     double *dma = staged ? slot(nchunk) : host + z0 * 8;   // where this chunk's DMA copy reads or writes
     if (upload) {
@@ -547,16 +559,16 @@ static int transfer(mgpu_solver *h, double *host, const void *dev_in, void *dev_
       if (staged) {
         CK(cudaEventRecord(h->xfer_ev[nchunk % 2], h->stream));
         if (nchunk >= 1) {   // the previous chunk, from its slot into the caller's buffer
-          const long long zp = z0 - h->staging_zones;
+          const long long zp = z0 - chunk;
           CK(cudaEventSynchronize(h->xfer_ev[(nchunk - 1) % 2]));
-          h->pipe_pool->copy(host + zp * 8, slot(nchunk - 1), (size_t) h->staging_zones * 8 * sizeof(double));
+          h->pipe_pool->copy(host + zp * 8, slot(nchunk - 1), (size_t) chunk * 8 * sizeof(double));
         }
       }
     }
     ++nchunk;
   }
   if (staged && !upload && nchunk >= 1) {   // the last chunk
-    const long long zl = zbeg + (long long) (nchunk - 1) * h->staging_zones;
+    const long long zl = zbeg + (long long) (nchunk - 1) * chunk;
     CK(cudaEventSynchronize(h->xfer_ev[(nchunk - 1) % 2]));
     h->pipe_pool->copy(host + zl * 8, slot(nchunk - 1), (size_t) (nz - zl) * 8 * sizeof(double));
   }
