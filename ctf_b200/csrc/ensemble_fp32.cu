@@ -9,8 +9,12 @@
 #ifndef MGPU_HLLD_MINB
 #define MGPU_HLLD_MINB 6
 #endif
+// zone c2p at 8 blocks, 64 registers (the FP64 state is live only through one or two Newton
+// steps): 160^3 lean c2p per RK3 step 0.68 / 0.62 / 0.56 ms at 5 / 6 / 8 blocks
 #ifdef MGPU_C2P_MINB_OVERRIDE
 #define MGPU_C2P_MINB MGPU_C2P_MINB_OVERRIDE
+#else
+#define MGPU_C2P_MINB 8
 #endif
 #ifdef MGPU_TC_CTAS_OVERRIDE
 #define MGPU_TC_CTAS_PER_SM MGPU_TC_CTAS_OVERRIDE

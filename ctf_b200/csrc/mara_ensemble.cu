@@ -481,7 +481,7 @@ int mgpu_ensemble_create(const mgpu_config *cfg, int nd, int nboxes, const int *
   e->launch.zone_tile = 1024;
   e->launch.face_tile = 512;
   e->launch.zone_ctas_per_sm = 8;
-  e->launch.face_ctas_per_sm = fp32(e) ? 4 : 3;
+  e->launch.face_ctas_per_sm = fp32(e) ? 5 : 3;
   e->launch.c2p_ctas_per_sm = 8;
   if (build_maps(e)) {
     fprintf(stderr, "[mgpu] ensemble: %s\n", e->err.c_str());

@@ -242,6 +242,7 @@ __global__ void __launch_bounds__(128) k_ctu_predict(Grid g, StateCPtr<T> U, con
   warp_add_int(&ctl->ctu_err[1], bad);
   warp_add_int(&ctl->ctu_err[2], c2p_bad);
   warp_add(&stat_slot(ctl).c2p_calls, calls);
+  warp_add(&stat_slot(ctl).predict_calls, calls);
   warp_add(&stat_slot(ctl).c2p_iters, iters);
 }
 

@@ -84,7 +84,7 @@ __global__ void __launch_bounds__(256) k_ens_p2c(const BoxDev *boxes, const int2
 
 // uin: 0 reads U0, 1 reads U1
 template <class T>
-__global__ void __launch_bounds__(128) k_ens_c2p(const BoxDev *boxes, const int2 *map, long long ntiles, int tile,
+__global__ void __launch_bounds__(128, MGPU_C2P_MINB) k_ens_c2p(const BoxDev *boxes, const int2 *map, long long ntiles, int tile,
                                                  PhysParams pp, int stage, int uin, int zero_guess, int final,
                                                  int ereset, double preset, double dreset)
 {

@@ -523,18 +523,68 @@ __device__ __forceinline__ int c2p_anton2dzw(const C2PState &s, double Z, double
   return c2p_reconstruct(s, Z, W, P);
 }
 
+// An approximate reciprocal, also in the translation units built without fast math.
+__device__ __forceinline__ float rcp32(float x) { return __fdividef(1.f, x); }
+
+// The Anton et al. iteration in FP32 to a step of 1e-6, from and to (Z, W); E = tau + D.  Non-zero
+// when it does not converge in `limit` iterations.
+__device__ __forceinline__ int c2p_newton32(float D, float E, float S2, float B2, float BS2, float gamf, float &Z,
+                                            float &W, int &iters, int limit)
+{
+  float iW = rcp32(W), iZ = rcp32(Z);
+  iters = 0;
+#pragma unroll 1
+  for (;;) {
+    const float W2 = W * W, iW2 = iW * iW, iW3 = iW2 * iW, iZ2 = iZ * iZ, iZ3 = iZ2 * iZ;
+    const float T = BS2 * iZ2;
+    const float BZ = B2 + Z, u2 = (W2 - 1.f) * iW2;
+    const float Pre = (Z * iW2 - D * iW) * gamf;
+    const float f0Z = 2.f * BZ * (BS2 * iZ3 + u2);
+    const float f0W = 2.f * BZ * BZ * iW3;
+    const float f1Z = 1.f + BS2 * iZ3 - gamf * iW2;
+    const float f1W = (B2 + (2.f * Z - D * W) * gamf) * iW3;
+    const float f0 = BZ * BZ * u2 - (2.f * Z + B2) * T - S2;
+    const float f1 = Z + B2 - E - Pre - 0.5f * B2 * iW2 - 0.5f * T;
+    const float idet = rcp32(f0Z * f1W - f0W * f1Z);
+    const float dZ = -(f1W * f0 - f0W * f1) * idet;
+    const float dW = -(f0Z * f1 - f1Z * f0) * idet;
+    const float Zn = fabsf(Z + dZ);
+    Z = (Zn < 1e20f) ? Zn : Z;
+    W = fminf(fmaxf(W + dW, 1.f), 1e12f);
+    iZ = rcp32(Z);
+    iW = rcp32(W);
+    const float err = fabsf(dZ * iZ) + fabsf(dW * iW);
+    ++iters;
+    if (!(err > 1e-6f)) return err == err ? 0 : 1;
+    if (iters == limit) return 1;
+  }
+}
+
 // The same Anton et al. Newton iteration with the divisions replaced by three reciprocals
 // per iteration (1/W, 1/Z, 1/det); algebraically identical, rounded differently.  Used by
 // the FP32-bulk path, whose c2p is an FP64 polish compared with the FP64 path rather than
-// the reference's bit pattern.
+// the reference's bit pattern.  The start is first brought to FP32 accuracy by the same
+// iteration in FP32 (five iterations from the estimate, at a quarter of their FP64 cost); a
+// first FP64 step below 1e-6 then leaves an error of its square, the 1e-12 the iteration asks
+// for, and ends it.  160^3 lean c2p: 0.82 -> 0.56 ms per RK3 step.
 __device__ __forceinline__ int c2p_anton2dzw_fast(const C2PState &s, double Z, double W, double *P, int &iters)
 {
   const double D = s.D, B2 = s.B2, BS2 = s.BS2, S2 = s.S2, gamf = s.gamf, Tau = s.Tau;
   const double iD = 1.0 / D;
+  int it32 = 0;
+  double tol = 1e-12;
+  {
+    float z = float(Z), w = float(W);
+    if (c2p_newton32(float(D), float(D + Tau), float(S2), float(B2), float(BS2), float(gamf), z, w, it32, 12) == 0) {
+      Z = z;
+      W = w;
+      tol = 1e-6;
+    }
+  }
   double iW = 1.0 / W, iZ = 1.0 / Z;
   double error = 1.0;
-  iters = 0;
-  while (error > 1e-12) {
+  iters = it32;
+  for (; error > tol; tol = 1e-12) {
     const double W2 = W * W, Z2 = Z * Z, Z3 = Z * Z2;
     const double iW2 = iW * iW, iW3 = iW2 * iW, iZ2 = iZ * iZ, iZ3 = iZ2 * iZ;
     const double Pre = D * iW * (Z * iD * iW - 1.0) * gamf;
@@ -558,8 +608,10 @@ __device__ __forceinline__ int c2p_anton2dzw_fast(const C2PState &s, double Z, d
     iZ = 1.0 / Z;
     iW = 1.0 / W;
     error = fabs(dZ * iZ) + fabs(dW * iW);
-    if (++iters == 250) return C2P_MAXITER;
+    if (!(error > tol)) break;
+    if (++iters >= 250) return C2P_MAXITER;
   }
+  ++iters;
   return c2p_reconstruct_fast(s, Z, W, iZ, iW, iD, P);
 }
 
@@ -1247,10 +1299,11 @@ __device__ __forceinline__ int hlld_newton(const HlldEqn<T> &q, T &x)
 // at the starting pressure, then inverse interpolation through the points already there --
 // Newton's first step and about its second from three evaluations, where the central
 // differences of each Newton iteration take three -- and as in hlld_newton a last step from the
-// point whose residual passes.  Faces on which this does not contract at once (a residual that
-// does not fall, NaN, not below 1e-6 after seven evaluations) run hlld_newton from the start, out of line,
-// so the face keeps the reference's outcome there.  On turbulence faces Newton takes 6 to 12
-// evaluations and this 4 (measured on 240,000 faces; the roots agree to 1e-14 of p).
+// point whose residual passes.  Faces on which the residual does not fall twentyfold in the
+// first step and fiftyfold in the later ones (or is NaN) run hlld_newton from the start, out of
+// line, and keep the reference's outcome: eq. 48 has other roots, and without this bound one
+// face in 10^8 took one.  Newton takes 6 to 12 evaluations on turbulence faces and this 4 or 5
+// (360,000 faces: fluxes within 1e-14 on 99.9%, the same branch on all).
 struct HlldRoot {
   double p;
   int err;
@@ -1272,7 +1325,7 @@ __device__ __forceinline__ int hlld_solve(const HlldEqn<double> &q, bool direct,
 {
   using Tol = RmhdTol<double>;
   const double dp = Tol::jac_dp;
-  double x0 = p, y0 = 0.0, s0 = 0.0;     // the start, its residual and dx/dy
+  double x0 = p, y0 = 0.0, s0 = 0.0, sl = 0.0;   // the start, its residual and dx/dy; the latest dx/dy
   double x1 = 0.0, y1 = 0.0;             // the latest point
   bool last = direct;
 #pragma unroll 1
@@ -1287,19 +1340,22 @@ __device__ __forceinline__ int hlld_solve(const HlldEqn<double> &q, bool direct,
     }
     bool ok = true;
     if (it == 1) {
-      s0 = dp / (y - y0);
+      sl = s0 = dp / (y - y0);
       x1 = x0;
       y1 = y0;
       p = x0 - s0 * y0;
     } else {
-      ok = fabs(y) <= 0.02 * fabs(y1) || fabs(y) <= Tol::newton_eps;
+      ok = fabs(y) <= (it == 2 ? 0.05 : 0.02) * fabs(y1) || fabs(y) <= Tol::newton_eps;
       double step;
       if (it == 2) {
         const double t = y0 / (y0 - y);
         step = s0 * y * t * t;
       } else {
-        step = y * (p - x1) / (y - y1);
+        // below 1e-8 the residuals' rounding would enter the secant: keep the last slope
+        if (fabs(y1) >= 1e-8) sl = (p - x1) / (y - y1);
+        step = sl * y;
       }
+      if (it == 2 && fabs(y0) >= 1e-8) sl = (p - x0) / (y - y0);
       x1 = p;
       y1 = y;
       p -= step;
@@ -1471,9 +1527,6 @@ static __device__ __noinline__ HllGuess64 hll_guess64(PhysParams pp, HllState64 
   return o;
 }
 
-// An approximate reciprocal, also in the translation units built without fast math.
-__device__ __forceinline__ float rcp32(float x) { return __fdividef(1.f, x); }
-
 // Total pressure of the HLL state, the first pressure guess, by the Anton et al. 2-D Newton in
 // FP32 from (Z, W) of the average face state, to a step of 1e-6 (the guess only seeds the
 // secants, and is kept in FP32): U as D, E, S0..S2, Bx, B1, B2.  Non-zero when the state fails
@@ -1491,36 +1544,8 @@ __device__ __forceinline__ int hll_pressure32(float gamma, float pfloor, float D
   const float B2 = Bx * Bx + B1 * B1 + B2_ * B2_;
   const float BS = Bx * S0 + B1 * S1 + B2_ * S2_;
   const float BS2 = BS * BS;
-  const float iD = rcp32(D);
-  float iW = rcp32(W), iZ = rcp32(Z);
-#pragma unroll 1
-  for (;;) {
-    const float W2 = W * W, iW2 = iW * iW, iW3 = iW2 * iW, iZ2 = iZ * iZ, iZ3 = iZ2 * iZ;
-    const float T = BS2 * iZ2;
-    const float BZ = B2 + Z, u2 = (W2 - 1.f) * iW2;
-    const float Pre = (Z * iW2 - D * iW) * gamf;
-    const float f0Z = 2.f * BZ * (BS2 * iZ3 + u2);
-    const float f0W = 2.f * BZ * BZ * iW3;
-    const float f1Z = 1.f + BS2 * iZ3 - gamf * iW2;
-    const float f1W = (B2 + (2.f * Z - D * W) * gamf) * iW3;
-    const float f0 = BZ * BZ * u2 - (2.f * Z + B2) * T - S2;
-    const float f1 = Z + B2 - E - Pre - 0.5f * B2 * iW2 - 0.5f * T;
-    const float idet = rcp32(f0Z * f1W - f0W * f1Z);
-    const float dZ = -(f1W * f0 - f0W * f1) * idet;
-    const float dW = -(f0Z * f1 - f1Z * f0) * idet;
-    const float Zn = fabsf(Z + dZ);
-    Z = (Zn < 1e20f) ? Zn : Z;
-    W = fminf(fmaxf(W + dW, 1.f), 1e12f);
-    iZ = rcp32(Z);
-    iW = rcp32(W);
-    const float err = fabsf(dZ * iZ) + fabsf(dW * iW);
-    ++iters;
-    if (!(err > 1e-6f)) {
-      if (!(err == err)) return 1;
-      break;
-    }
-    if (iters == 32) return 1;
-  }
+  if (c2p_newton32(D, E, S2, B2, BS2, gamf, Z, W, iters, 32)) return 1;
+  const float iD = rcp32(D), iW = rcp32(W), iZ = rcp32(Z);
   const float r = D * iW;
   float p = r * (Z * iD * iW - 1.f) * gamf;
   if (pfloor > 0.f && p < pfloor) p = pfloor;

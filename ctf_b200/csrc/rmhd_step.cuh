@@ -186,8 +186,8 @@ __device__ __forceinline__ void c2p_finish(const Grid &g, T *PA, StatePtr<T> Pn,
     StatSlot &st = stat_slot(ctl);
     warp_add(&st.c2p_calls, 1u);
     warp_add(&st.c2p_iters, (unsigned) tally.iters);
-    if (tally.attempts >= 1 && tally.attempts <= 5) warp_add(&st.c2p_attempt[tally.attempts], 1u);
-    warp_add(&st.c2p_failed, err ? 1u : 0u);
+    if (tally.attempts != 1) warp_add(&st.c2p_attempt[tally.attempts], 1u);   // [1] is the rest
+    if (err) warp_add(&st.c2p_failed, 1u);
   }
   if (err) {
     if (ereset) {   // emergency reset of the failed zone
@@ -209,29 +209,41 @@ __device__ __forceinline__ void c2p_finish(const Grid &g, T *PA, StatePtr<T> Pn,
   // the failure mask of this c2p at the zone and its images (an emergency reset clears it)
   unsigned char *const fm = counted ? ctl->fmask : nullptr;
   const unsigned char failed = (unsigned char) (err && !ereset);
+  const auto store = [&](long long w) {
+    if (fm) fm[w] = failed;
+    if (final == C2P_CLOSING || final == C2P_DIFFUSE) {
+#pragma unroll
+      for (int q = 0; q < 5; ++q) Pn.bulk[q * g.cs + w] = T(p[q]);
+#pragma unroll
+      for (int q = 0; q < 3; ++q) Pn.B[q * g.cs + w] = p[5 + q];
+    } else {
+#pragma unroll
+      for (int q = 0; q < 8; ++q) PA[q * g.cs + w] = T(p[q]);
+      if (final == C2P_LEAN_CLOSING) {   // the field of the register about to be committed
+#pragma unroll
+        for (int q = 0; q < 3; ++q) Pn.B[q * g.cs + w] = u[5 + q];
+      }
+    }
+  };
+  // a zone further than ng from every face has no image
+  const int m[3] = {i, j, k};
+  bool inside = true;
+#pragma unroll
+  for (int d = 0; d < 3; ++d) inside = inside && (d >= g.nd || (m[d] >= 2 * g.ng && m[d] < g.n[d]));
+  if (inside) {
+    store(((long long) i * g.G[1] + j) * g.G[2] + k);
+    return;
+  }
   int pi[3], pj[3], pk[3];
   const int ni = images_1d(i, g.n[0], g.ng, self_periodic(g, 0), pi);
   const int nj = images_1d(j, g.n[1], g.ng, self_periodic(g, 1), pj);
   const int nk = images_1d(k, g.n[2], g.ng, self_periodic(g, 2), pk);
+#pragma unroll 1
   for (int a = 0; a < ni; ++a)
+#pragma unroll 1
     for (int b = 0; b < nj; ++b)
-      for (int c = 0; c < nk; ++c) {
-        const long long w = ((long long) pi[a] * g.G[1] + pj[b]) * g.G[2] + pk[c];
-        if (fm) fm[w] = failed;
-        if (final == C2P_CLOSING || final == C2P_DIFFUSE) {
-#pragma unroll
-          for (int q = 0; q < 5; ++q) Pn.bulk[q * g.cs + w] = T(p[q]);
-#pragma unroll
-          for (int q = 0; q < 3; ++q) Pn.B[q * g.cs + w] = p[5 + q];
-        } else {
-#pragma unroll
-          for (int q = 0; q < 8; ++q) PA[q * g.cs + w] = T(p[q]);
-          if (final == C2P_LEAN_CLOSING) {   // the field of the register about to be committed
-#pragma unroll
-            for (int q = 0; q < 3; ++q) Pn.B[q * g.cs + w] = u[5 + q];
-          }
-        }
-      }
+#pragma unroll 1
+      for (int c = 0; c < nk; ++c) store(((long long) pi[a] * g.G[1] + pj[b]) * g.G[2] + pk[c]);
 }
 
 // The conserved input of a c2p launch: U, or in the lean layout one of the two conserved

@@ -39,12 +39,15 @@ constexpr int MAX_STAGES = 4;
 // to slot b % STAT_SLOTS and the host sums the slots.  With one copy every warp's atomic went
 // to the same cache line and they serialised (2 ms per 256^3 step in the zone c2p alone).
 constexpr int STAT_SLOTS = 32;
+// c2p_attempt[1], the common case, is not counted: it is what c2p_calls leaves after the other
+// outcomes ([0]: the state failed its checks before any attempt) and the predictor's calls.
 struct StatSlot {
   unsigned long long c2p_calls, c2p_iters, c2p_attempt[6];
   unsigned long long face_c2p_calls, face_c2p_iters;
   unsigned long long hlld_ok, hlld_hllc, pcm_retry;
   unsigned long long c2p_failed;   // zone c2p calls that failed every rung (reset or not)
-  unsigned long long pad[2];       // 128 bytes
+  unsigned long long predict_calls;   // those of c2p_calls made by the CTU-Hancock predictor
+  unsigned long long pad;             // 128 bytes
 };
 
 // What a c2p launch reads, where it writes and which counter its failures go to.
@@ -102,7 +105,12 @@ inline StatSlot stat_sum(const Ctl &c)
     t.hlld_hllc += s.hlld_hllc;
     t.pcm_retry += s.pcm_retry;
     t.c2p_failed += s.c2p_failed;
+    t.predict_calls += s.predict_calls;
   }
+  t.c2p_attempt[1] = t.c2p_calls - t.predict_calls;
+  for (int a = 0; a < 6; ++a)
+    if (a != 1) t.c2p_attempt[1] -= t.c2p_attempt[a];
+  t.c2p_attempt[0] = 0;
   return t;
 }
 
