@@ -112,10 +112,11 @@ inline cudaError_t launch_lean_phase(const AdvanceArgs &A, int phase, int s)
                                                      A.preset, A.dreset, phase == PH_C2P_SHELL ? 1 : 2);
   } else if (phase == PH_FLUX_UPDATE) {
     const StageKind kind = stage_kind(A.rk, s);
-    const LeanCombine c = lean_combine(kind.combine);
+    const double dx[3] = {g.dx, g.dy, g.dz};
     for (int d = 1; d <= 3; ++d) {
       ProfScope ps(pr, st, KC_FLUX, nwin);
-      launch_lean_sweep<T>(g, d, A.pp.riemann, st, PA, UA, UB, Bf, c, A.pp, A.ctl, s);
+      launch_lean_sweep<T>(g, d, A.pp.riemann, st, PA, UA, UB, Bf, lean_combine<T>(kind.combine, dx[d - 1]), A.pp,
+                           A.ctl, s);
     }
     ProfScope ps(pr, st, KC_UPDATE, nwin);
     const unsigned zb = 256;

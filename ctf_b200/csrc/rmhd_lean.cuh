@@ -29,19 +29,21 @@
 
 namespace mgpu {
 
-struct LeanCombine {   // U1 = alpha U0 + beta U1 + gamma dt L
-  double alpha, beta, gamma;
-  int first;           // 1: the x sweep applies the combine (0: y/z sweeps add)
+// U1 = alpha U0 + beta U1 + gamma dt L, L over zones of width 1 / inv_dx: rounded to the kernels'
+// type on the host, so that the kernels take them from the constant bank as they are.
+template <class T> struct LeanCombine {
+  T alpha, beta, gamma, inv_dx;
   int euler;           // beta == 0: U1's previous contents are not read
 };
 
-__host__ __device__ inline LeanCombine lean_combine(int combine)
+template <class T> inline LeanCombine<T> lean_combine(int combine, double dx)
 {
+  const T inv = T(1.0 / dx);
   switch (combine) {
-  case COMB_RK2_2: return {0.5, 0.5, 0.5, 1, 0};
-  case COMB_RK3_2: return {0.75, 0.25, 0.25, 1, 0};
-  case COMB_RK3_3: return {1.0 / 3.0, 2.0 / 3.0, 2.0 / 3.0, 1, 0};
-  default: return {1.0, 0.0, 1.0, 1, 1};
+  case COMB_RK2_2: return {T(0.5), T(0.5), T(0.5), inv, 0};
+  case COMB_RK3_2: return {T(0.75), T(0.25), T(0.25), inv, 0};
+  case COMB_RK3_3: return {T(1.0 / 3.0), T(2.0 / 3.0), T(2.0 / 3.0), inv, 0};
+  default: return {T(1.0), T(0.0), T(1.0), inv, 1};
   }
 }
 
@@ -62,18 +64,17 @@ __host__ __device__ constexpr int bf_slot(int dim, int b)
 // Adds one direction's flux difference to interior zone z of the register (bulk components).
 template <class T>
 __device__ __forceinline__ void lean_accumulate(const Grid &g, StatePtr<T> U0, StatePtr<T> U1, long long z,
-                                                const T *Flo, const T *Fhi, T inv_dx, const LeanCombine &c, T dt,
-                                                bool first)
+                                                const T *Flo, const T *Fhi, const LeanCombine<T> &c, T dt, bool first)
 {
-  const T gdt = T(c.gamma) * dt;
+  const T gdt = c.gamma * dt;
 #pragma unroll
   for (int q = 0; q < 5; ++q) {
-    const T L = -(Fhi[q] - Flo[q]) * inv_dx;
+    const T L = -(Fhi[q] - Flo[q]) * c.inv_dx;
     T *u1 = U1.bulk + q * g.cs + z;
     if (first) {
       const T u0 = U0.bulk[q * g.cs + z];
       const T prev = c.euler ? T(0) : *u1;
-      *u1 = T(c.alpha) * u0 + T(c.beta) * prev + gdt * L;
+      *u1 = c.alpha * u0 + c.beta * prev + gdt * L;
     } else {
       *u1 += gdt * L;
     }
@@ -88,10 +89,49 @@ __device__ __forceinline__ void lean_accumulate(const Grid &g, StatePtr<T> U0, S
 // Each zone is reconstructed once, both its faces together: the upper face value waits in
 // shared memory for the next face.  Consecutive threads take consecutive k, so every load and
 // store is coalesced.
-template <class T, int dim, int RS>
+//
+// The next zone's leading row is new to the chip: it is brought closer while the face's Riemann
+// problem is solved, which takes longer than a read of memory.  PLM asks for it to be in L2; its
+// other two rows are still in L1.  FP32 WENO5 keeps the stencil's five rows and the coming one
+// in a ring in shared memory (24 KB per CTA; the 123 KB of five rows of a full SM do not stay in
+// L1), copies the coming row into it, and has kernels of its own (W5), by which the others come
+// out shorter, too.  160^3, RK3 WENO5, nine sweeps: 4.60 ms before, 4.37 with the row asked for,
+// 4.16 with the ring; RK2 PLM, six sweeps: 2.33, 2.25, and 2.22 in kernels without WENO5 (2.30
+// with a ring of four rows).  FP64 has one kernel and asks for the row.
+constexpr int LEAN_ROW = 8 * 128, LEAN_RING = 6 * LEAN_ROW;   // entries
+template <class T> __host__ __device__ constexpr bool lean_split() { return sizeof(T) == 4; }
+__device__ __forceinline__ int lean_ring_wrap(int off)
+{
+  return off < 0 ? off + LEAN_RING : off >= LEAN_RING ? off - LEAN_RING : off;
+}
+
+// Starts copying the eight components at a into this thread's entries of a ring row.  A thread
+// reads back its own copies only, so that waiting for them needs no barrier.
+__device__ __forceinline__ void lean_fetch(float *row, const float *a, long long cs)
+{
+  const unsigned s = (unsigned) __cvta_generic_to_shared(row);
+#pragma unroll
+  for (int c = 0; c < 8; ++c)
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(s + c * 512), "l"(a + c * cs) : "memory");
+  asm volatile("cp.async.commit_group;" ::: "memory");
+}
+__device__ __forceinline__ void lean_fetch(double *, const double *, long long) {}
+
+// zone_states with WENO5 from the ring; row[0..4]: the entries of the stencil's rows.
+template <class T, int RS>
+__device__ __forceinline__ void lean_ring_states(const PhysParams &pp, int dim, const T *const *row, T *lo, T *hi)
+{
+#pragma unroll
+  for (int c = 0; c < 8; ++c) {
+    const int q = slot_of<T, RS>(dim, c), e = c * 128;
+    weno5_zone(pp.is_mode, T(pp.sz10A), row[0][e], row[1][e], row[2][e], row[3][e], row[4][e], lo[q], hi[q]);
+  }
+}
+
+template <class T, int dim, int RS, bool W5>
 __global__ void __launch_bounds__(128, flux_minb<RS>()) k_lean_sweep(Grid g, const T *__restrict__ PA, StatePtr<T> UA,
                                                                     StatePtr<T> UB, T *__restrict__ Bf,
-                                                                    LeanCombine c, PhysParams pp, Ctl *ctl, int stage,
+                                                                    LeanCombine<T> c, PhysParams pp, Ctl *ctl, int stage,
                                                                     int chunk_len)
 {
   static_assert(dim == 1 || dim == 2, "x or y sweep");
@@ -113,6 +153,8 @@ __global__ void __launch_bounds__(128, flux_minb<RS>()) k_lean_sweep(Grid g, con
   FluxTally ft{0, 0, 0, 0, 0};
   __shared__ T flo[128][5];   // the carried lower-face flux of each thread
   __shared__ T up[8][128];    // the carried upper-face state of the face's lower zone
+  __shared__ T ring_rows[W5 ? LEAN_RING : 1];
+  T *const ring = ring_rows + threadIdx.x;
   __shared__ T cols[column_entries<T, RS>() * 128];
   if (t < ncol * nchunk) {
     const int chunk = (int) (t / ncol);
@@ -125,19 +167,36 @@ __global__ void __launch_bounds__(128, flux_minb<RS>()) k_lean_sweep(Grid g, con
     const long long base = (long long) ca * g.s[oa] + k;   // zone (0 along dim, ca, k)
     const int m0 = g.ng + mlo + chunk * chunk_len;
     const int m1 = min(m0 + chunk_len, g.ng + mhi);
-    const T inv_dx = T(1.0 / (dim == 1 ? g.dx : g.dy));
     const T dt = T(ctl->dt);
     T *slot0 = Bf + (long long) bf_slot(dim, dim == 1 ? By : Bx) * g.cs;
     T *slot1 = Bf + (long long) bf_slot(dim, Bz) * g.cs;
+    int mid = 2 * LEAN_ROW;      // ring offset of the zone being reconstructed
     {
       T lo[8], hi[8];
-      zone_states<T, RS>(g, PA, pp, dim, base + (long long) (m0 - 1) * S, lo, hi);
+      const long long z = base + (long long) (m0 - 1) * S;
+      if constexpr (W5) {
+        for (int o = -2; o <= 3; ++o) lean_fetch(ring + mid + o * LEAN_ROW, PA + z + o * S, g.cs);
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        const T *row[5];
+#pragma unroll
+        for (int o = 0; o < 5; ++o) row[o] = ring + o * LEAN_ROW;
+        lean_ring_states<T, RS>(pp, dim, row, lo, hi);
+      } else zone_states<T, RS, lean_split<T>() ? ZONE_NOT_WENO5 : ZONE_ANY>(g, PA, pp, dim, z, lo, hi);
 #pragma unroll
       for (int q = 0; q < 8; ++q) up[q][threadIdx.x] = hi[q];
     }
 #pragma unroll 1
     for (int m = m0 - 1; m < m1; ++m) {   // face between zones m and m + 1
       const long long f = base + (long long) m * S;
+      if constexpr (W5) {
+        mid = lean_ring_wrap(mid + LEAN_ROW);
+        // into the entries of the last zone's lowest row
+        if (m + 1 < m1) lean_fetch(ring + lean_ring_wrap(mid + 3 * LEAN_ROW), PA + f + 4 * S, g.cs);
+      } else if (m + 1 < m1) {
+        const T *next = PA + f + (pp.recon == RECON_PCM ? 2 : pp.recon == RECON_PLM ? 3 : 4) * S;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) asm volatile("prefetch.global.L2 [%0];" ::"l"(next + q * g.cs));
+      }
       if (m >= m0 && interior) {   // the register entries this face updates: into L2 while HLLD runs
 #pragma unroll
         for (int q = 0; q < 5; ++q) {
@@ -148,7 +207,14 @@ __global__ void __launch_bounds__(128, flux_minb<RS>()) k_lean_sweep(Grid g, con
       T Pl[8], Pr[8], hi[8], Ff[8], Fo[8];
 #pragma unroll
       for (int q = 0; q < 8; ++q) Pl[q] = up[q][threadIdx.x];
-      zone_states<T, RS>(g, PA, pp, dim, f + S, Pr, hi);
+      if constexpr (W5) {
+        if (m + 1 < m1) asm volatile("cp.async.wait_group 1;" ::: "memory");
+        else asm volatile("cp.async.wait_group 0;" ::: "memory");
+        const T *row[5];
+#pragma unroll
+        for (int o = 0; o < 5; ++o) row[o] = ring + lean_ring_wrap(mid + (o - 2) * LEAN_ROW);
+        lean_ring_states<T, RS>(pp, dim, row, Pr, hi);
+      } else zone_states<T, RS, lean_split<T>() ? ZONE_NOT_WENO5 : ZONE_ANY>(g, PA, pp, dim, f + S, Pr, hi);
 #pragma unroll
       for (int q = 0; q < 8; ++q) up[q][threadIdx.x] = hi[q];
       solve_face<T, RS, true>(g, PA, pp, dim, f, Pl, Pr, ml, ft, Ff, cols + threadIdx.x);
@@ -158,7 +224,7 @@ __global__ void __launch_bounds__(128, flux_minb<RS>()) k_lean_sweep(Grid g, con
         slot0[f] = Fo[dim == 1 ? By : Bx];
         slot1[f] = Fo[Bz];
       }
-      if (m >= m0 && interior) lean_accumulate<T>(g, U0, U1, f, flo[threadIdx.x], Fo, inv_dx, c, dt, dim == 1);
+      if (m >= m0 && interior) lean_accumulate<T>(g, U0, U1, f, flo[threadIdx.x], Fo, c, dt, dim == 1);
 #pragma unroll
       for (int q = 0; q < 5; ++q) flo[threadIdx.x][q] = Fo[q];
     }
@@ -172,10 +238,10 @@ __global__ void __launch_bounds__(128, flux_minb<RS>()) k_lean_sweep(Grid g, con
 // (both its faces), solves the face below it with the upper state of thread t - 1's zone, and
 // from the fluxes of threads t - 1 and t updates the zone below it; so each CTA solves 127
 // faces and updates 126 zones, its first face being the previous CTA's last.
-template <class T, int RS>
+template <class T, int RS, bool W5>
 __global__ void __launch_bounds__(128, flux_minb<RS>()) k_lean_sweep_z(Grid g, const T *__restrict__ PA, StatePtr<T> UA,
                                                                       StatePtr<T> UB, T *__restrict__ Bf,
-                                                                      LeanCombine c, PhysParams pp, Ctl *ctl,
+                                                                      LeanCombine<T> c, PhysParams pp, Ctl *ctl,
                                                                       int stage)
 {
   if (stage_failed(ctl, stage + 1)) return;
@@ -208,7 +274,7 @@ __global__ void __launch_bounds__(128, flux_minb<RS>()) k_lean_sweep_z(Grid g, c
       for (int r = 0; r < 5; ++r) asm volatile("prefetch.global.L2 [%0];" ::"l"(U1.bulk + r * g.cs + z - 1));
     }
     T hi[8];
-    zone_states<T, RS>(g, PA, pp, 3, z, Pr, hi);
+    zone_states<T, RS, W5 ? ZONE_WENO5 : lean_split<T>() ? ZONE_NOT_WENO5 : ZONE_ANY>(g, PA, pp, 3, z, Pr, hi);
 #pragma unroll
     for (int r = 0; r < 8; ++r) up[r][threadIdx.x] = hi[r];
   }
@@ -235,7 +301,7 @@ __global__ void __launch_bounds__(128, flux_minb<RS>()) k_lean_sweep_z(Grid g, c
       lo[r] = fs[r][threadIdx.x - 1];
       hi[r] = fs[r][threadIdx.x];
     }
-    lean_accumulate<T>(g, U0, U1, z - 1, lo, hi, T(1.0 / g.dz), c, T(ctl->dt), false);
+    lean_accumulate<T>(g, U0, U1, z - 1, lo, hi, c, T(ctl->dt), false);
   }
   flux_block_finish(double(ml), ft, ctl, RS == RIEMANN_HLLD);
 }
@@ -395,14 +461,19 @@ inline int lean_chunk(long long ncol, int n, long long resident_threads)
 
 template <class T>
 inline void launch_lean_sweep(const Grid &g, int dim, int rs, cudaStream_t st, const T *PA, StatePtr<T> UA,
-                              StatePtr<T> UB, T *Bf, const LeanCombine &c, const PhysParams &pp, Ctl *ctl, int s)
+                              StatePtr<T> UB, T *Bf, const LeanCombine<T> &c, const PhysParams &pp, Ctl *ctl, int s)
 {
   const unsigned blk = 128;
+  const bool w5 = lean_split<T>() && pp.recon == RECON_WENO5;
   if (dim == 3) {
     const long long total = (long long) (win_fhi(g) - win_flo(g)) * (g.n[1] + 2) * (g.n[2] + 2);
     const unsigned grid = (unsigned) ((total + 125) / 126);
 #define MGPU_LEANZ_CASE(R) \
-  if (rs == R) { k_lean_sweep_z<T, R><<<grid, blk, 0, st>>>(g, PA, UA, UB, Bf, c, pp, ctl, s); return; }
+  if (rs == R) {                                                                                           \
+    if (w5) k_lean_sweep_z<T, R, lean_split<T>()><<<grid, blk, 0, st>>>(g, PA, UA, UB, Bf, c, pp, ctl, s); \
+    else k_lean_sweep_z<T, R, false><<<grid, blk, 0, st>>>(g, PA, UA, UB, Bf, c, pp, ctl, s);              \
+    return;                                                                                                \
+  }
     MGPU_LEANZ_CASE(RIEMANN_HLLD) MGPU_LEANZ_CASE(RIEMANN_HLLC) MGPU_LEANZ_CASE(RIEMANN_HLL)
 #undef MGPU_LEANZ_CASE
     return;
@@ -416,7 +487,11 @@ inline void launch_lean_sweep(const Grid &g, int dim, int rs, cudaStream_t st, c
   const long long nchunk = (nmarch + L - 1) / L;
   const unsigned grid = (unsigned) ((ncol * nchunk + blk - 1) / blk);
 #define MGPU_LEAN_CASE(D, R) \
-  if (dim == D && rs == R) { k_lean_sweep<T, D, R><<<grid, blk, 0, st>>>(g, PA, UA, UB, Bf, c, pp, ctl, s, L); return; }
+  if (dim == D && rs == R) {                                                                                     \
+    if (w5) k_lean_sweep<T, D, R, lean_split<T>()><<<grid, blk, 0, st>>>(g, PA, UA, UB, Bf, c, pp, ctl, s, L);   \
+    else k_lean_sweep<T, D, R, false><<<grid, blk, 0, st>>>(g, PA, UA, UB, Bf, c, pp, ctl, s, L);                \
+    return;                                                                                                      \
+  }
   MGPU_LEAN_CASE(1, RIEMANN_HLLD) MGPU_LEAN_CASE(2, RIEMANN_HLLD)
   MGPU_LEAN_CASE(1, RIEMANN_HLLC) MGPU_LEAN_CASE(2, RIEMANN_HLLC)
   MGPU_LEAN_CASE(1, RIEMANN_HLL) MGPU_LEAN_CASE(2, RIEMANN_HLL)

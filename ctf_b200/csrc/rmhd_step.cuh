@@ -420,8 +420,10 @@ __device__ __forceinline__ void face_states_column(const Grid &g, const T *__res
 }
 
 // Both face values of zone z along direction dim: lo toward z - S, hi toward z + S, which are
-// face_states' Pr of the face below and Pl of the face above.
-template <class T, int RS>
+// face_states' Pr of the face below and Pl of the face above.  which: the reconstructions that
+// pp may ask for, where the launch has chosen the kernel by them.
+enum { ZONE_ANY, ZONE_WENO5, ZONE_NOT_WENO5 };
+template <class T, int RS, int which = ZONE_ANY>
 __device__ __forceinline__ void zone_states(const Grid &g, const T *__restrict__ PA, const PhysParams &pp, int dim,
                                             long long z, T *lo, T *hi)
 {
@@ -433,9 +435,9 @@ __device__ __forceinline__ void zone_states(const Grid &g, const T *__restrict__
     const int q = slot_of<T, RS>(dim, c);                \
     expr;                                                \
   }
-  if (pp.recon == RECON_PCM) {
+  if (which != ZONE_WENO5 && pp.recon == RECON_PCM) {
     MGPU_ZONE_LOOP(lo[q] = hi[q] = a[0])
-  } else if (pp.recon == RECON_PLM) {
+  } else if (which == ZONE_NOT_WENO5 || (which == ZONE_ANY && pp.recon == RECON_PLM)) {
     const T theta = T(pp.theta);
     MGPU_ZONE_LOOP(plm_zone(theta, a[-S], a[0], a[S], lo[q], hi[q]))
   } else {
