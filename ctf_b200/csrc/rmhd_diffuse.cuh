@@ -78,7 +78,7 @@ __global__ void __launch_bounds__(256) k_diffuse_update(Grid g, StateCPtr<T> U0,
   const UpdateArgs a{COMB_EULER, 0.0};
   const StateCPtr<T> none{nullptr, nullptr};
   update_zone<T, ND>(g, a, U0, none, F, G, H, U1, StatePtr<T>{nullptr, nullptr}, none, none, none, 1.0,
-                     interior_zone(g, t));
+                     make_double3(1.0 / g.dx, 1.0 / g.dy, 1.0 / g.dz), interior_zone(g, t));
 }
 
 static __global__ void k_diffuse_begin(Ctl *ctl)

@@ -131,10 +131,12 @@ __global__ void __launch_bounds__(128, flux_minb<RS>()) k_ens_flux(const BoxDev 
 }
 
 // out: 0 writes U0, 1 writes U1; kout: -1 none, else K[kout] (RK4).  ND: the boxes' common
-// dimensionality.  At least MGPU_ENS_UPDATE_MINB resident blocks (an HBM-bound kernel wants
-// occupancy more than the loop-invariant box fields the compiler would otherwise hoist).
+// dimensionality.  At least MGPU_ENS_UPDATE_MINB resident blocks: with all of a zone's operands
+// read ahead, the registers to hold them are worth more than warps to wait with (40 FP32 2-D
+// Kelvin-Helmholtz boxes, 6 launches: 4 blocks .469 ms, 3 .422, 2 .383; read per component
+// with 4 blocks .626).
 #ifndef MGPU_ENS_UPDATE_MINB
-#define MGPU_ENS_UPDATE_MINB 4   // chosen by a sweep of 2-4
+#define MGPU_ENS_UPDATE_MINB 2
 #endif
 template <class T, int ND>
 __global__ void __launch_bounds__(256, MGPU_ENS_UPDATE_MINB) k_ens_update(const BoxDev *boxes, const int2 *map, long long ntiles,
@@ -153,11 +155,12 @@ __global__ void __launch_bounds__(256, MGPU_ENS_UPDATE_MINB) k_ens_update(const 
     const StateCPtr<T> K1 = box_cstate<T>(d.b.K_bulk[0], d.b.K_B[0]), K2 = box_cstate<T>(d.b.K_bulk[1], d.b.K_B[1]),
                        K3 = box_cstate<T>(d.b.K_bulk[2], d.b.K_B[2]);
     const double dt = d.ctl->dt;
+    const double3 inv = make_double3(1.0 / d.g.dx, 1.0 / d.g.dy, 1.0 / d.g.dz);
     for (int s = threadIdx.x; s < tile; s += blockDim.x) {
       const long long t = base + s;
       if (t < d.g.ninterior)
         update_zone<T, ND>(d.g, a, U0, U1, (const T *) d.b.F[0], (const T *) d.b.F[1], (const T *) d.b.F[2], Uout,
-                           Kout, K1, K2, K3, dt, interior_zone(d.g, t));
+                           Kout, K1, K2, K3, dt, inv, interior_zone(d.g, t));
     }
   }
 }

@@ -216,12 +216,13 @@ inline cudaError_t launch_phase(const AdvanceArgs &A, int phase, int s)
     ProfScope ps(pr, st, KC_UPDATE, g.ninterior);
     const StateCPtr<T> cU0{U0.bulk, U0.B}, cU1{U1.bulk, U1.B}, cK0{K[0].bulk, K[0].B}, cK1{K[1].bulk, K[1].B},
         cK2{K[2].bulk, K[2].B};
+    const double3 inv = make_double3(1.0 / g.dx, 1.0 / g.dy, 1.0 / g.dz);
     if (g.nd == 1)
-      k_update<T, 1><<<zgrid, zb, 0, st>>>(g, ua, cU0, cU1, F, G, H, Uout, Kout, cK0, cK1, cK2, A.ctl, s);
+      k_update<T, 1><<<zgrid, zb, 0, st>>>(g, ua, cU0, cU1, F, G, H, Uout, Kout, cK0, cK1, cK2, A.ctl, s, inv);
     else if (g.nd == 2)
-      k_update<T, 2><<<zgrid, zb, 0, st>>>(g, ua, cU0, cU1, F, G, H, Uout, Kout, cK0, cK1, cK2, A.ctl, s);
+      k_update<T, 2><<<zgrid, zb, 0, st>>>(g, ua, cU0, cU1, F, G, H, Uout, Kout, cK0, cK1, cK2, A.ctl, s, inv);
     else
-      k_update<T, 3><<<zgrid, zb, 0, st>>>(g, ua, cU0, cU1, F, G, H, Uout, Kout, cK0, cK1, cK2, A.ctl, s);
+      k_update<T, 3><<<zgrid, zb, 0, st>>>(g, ua, cU0, cU1, F, G, H, Uout, Kout, cK0, cK1, cK2, A.ctl, s, inv);
   } else if (phase == PH_COMMIT) {
     ProfScope ps(pr, st, KC_BEGIN, 1);
     k_commit<<<1, 32, 0, st>>>(A.ctl, ns);

@@ -660,37 +660,65 @@ __device__ __forceinline__ T combine_bulk(const UpdateArgs &a, T un, T us, T dt,
   }
 }
 
+// Zone z's bulk components 0..4: plain flux differences in T.  Here and in update_field everything
+// is read before anything is written: the compiler cannot tell the stored component from the next
+// one's operands, and would make the components' reads wait for one another, eight trips to
+// memory in a row where one is enough.  Per step, the update's launches: 96^3 FP32 RK2
+// 0.150 -> 0.117 ms, 160^3 FP32 RK3 0.92 -> 0.66, 96^3 FP64 RK3 0.367 -> 0.353.
 template <class T, int ND>
-__device__ __forceinline__ void update_zone(const Grid &g, const UpdateArgs &a, StateCPtr<T> Un, StateCPtr<T> Us,
+__device__ __forceinline__ void update_bulk(const Grid &g, const UpdateArgs &a, StateCPtr<T> Un, StateCPtr<T> Us,
                                             const T *__restrict__ F, const T *__restrict__ G,
                                             const T *__restrict__ H, StatePtr<T> Uout, StatePtr<T> Kout,
                                             StateCPtr<T> K1, StateCPtr<T> K2, StateCPtr<T> K3, double dtd,
                                             long long z)
 {
   const long long sx = g.s[0], sy = g.s[1], sz = g.s[2];
-  const double dx = g.dx, dy = g.dy, dz = g.dz;
-  const T dt = T(dtd);
-  const bool rk4 = a.combine >= COMB_RK4_K;
-  // bulk components 0..4: plain flux differences in T
+  const T dx = T(g.dx), dy = T(g.dy), dz = T(g.dz), dt = T(dtd);
+  const bool two = a.combine == COMB_RK2_2 || a.combine == COMB_RK3_2 || a.combine == COMB_RK3_3;
+  T un[5], us[5], L[5];
 #pragma unroll
   for (int q = 0; q < 5; ++q) {
-    T L;
+    un[q] = Un.bulk[q * g.cs + z];
+    us[q] = two ? Us.bulk[q * g.cs + z] : T(0);
+  }
+#pragma unroll
+  for (int q = 0; q < 5; ++q) {
+    const T *f = F + q * g.cs + z, *h = G + q * g.cs + z, *k = H + q * g.cs + z;
     if (ND == 1) {
-      L = -(F[q * g.cs + z] - F[q * g.cs + z - sx]) / T(dx);
+      L[q] = -(f[0] - f[-sx]) / dx;
     } else if (ND == 2) {
-      L = -(F[q * g.cs + z] - F[q * g.cs + z - sx]) / T(dx) - (G[q * g.cs + z] - G[q * g.cs + z - sy]) / T(dy);
+      L[q] = -(f[0] - f[-sx]) / dx - (h[0] - h[-sy]) / dy;
     } else {
-      L = -(F[q * g.cs + z] - F[q * g.cs + z - sx]) / T(dx) - (G[q * g.cs + z] - G[q * g.cs + z - sy]) / T(dy) -
-          (H[q * g.cs + z] - H[q * g.cs + z - sz]) / T(dz);
+      L[q] = -(f[0] - f[-sx]) / dx - (h[0] - h[-sy]) / dy - (k[0] - k[-sz]) / dz;
     }
-    const T un = Un.bulk[q * g.cs + z];
-    const T us = (a.combine == COMB_RK2_2 || a.combine == COMB_RK3_2 || a.combine == COMB_RK3_3) ? Us.bulk[q * g.cs + z] : T(0);
+  }
+#pragma unroll
+  for (int q = 0; q < 5; ++q) {
     T k1 = T(0), k2 = T(0), k3 = T(0), kk = T(0);
     if (a.combine == COMB_RK4_4) { k1 = K1.bulk[q * g.cs + z]; k2 = K2.bulk[q * g.cs + z]; k3 = K3.bulk[q * g.cs + z]; }
-    Uout.bulk[q * g.cs + z] = combine_bulk<T>(a, un, us, dt, L, &kk, k1, k2, k3);
-    if (rk4 && a.combine == COMB_RK4_K) Kout.bulk[q * g.cs + z] = kk;
+    Uout.bulk[q * g.cs + z] = combine_bulk<T>(a, un[q], us[q], dt, L[q], &kk, k1, k2, k3);
+    if (a.combine == COMB_RK4_K) Kout.bulk[q * g.cs + z] = kk;
   }
-  // magnetic components 5..7 in double, with the constrained-transport fluxes
+}
+
+// Zone z's field components 5..7 in double, with the constrained-transport fluxes.  inv: 1/dx,
+// 1/dy, 1/dz, for the FP32 bulk's form.
+template <class T, int ND>
+__device__ __forceinline__ void update_field(const Grid &g, const UpdateArgs &a, StateCPtr<T> Un, StateCPtr<T> Us,
+                                             const T *__restrict__ F, const T *__restrict__ G,
+                                             const T *__restrict__ H, StatePtr<T> Uout, StatePtr<T> Kout,
+                                             StateCPtr<T> K1, StateCPtr<T> K2, StateCPtr<T> K3, double dtd,
+                                             double3 inv, long long z)
+{
+  const long long sx = g.s[0], sy = g.s[1], sz = g.s[2];
+  const double dx = g.dx, dy = g.dy, dz = g.dz;
+  const bool two = a.combine == COMB_RK2_2 || a.combine == COMB_RK3_2 || a.combine == COMB_RK3_3;
+  double bn[3], bs[3];
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    bn[c] = Un.B[c * g.cs + z];
+    bs[c] = two ? Us.B[c * g.cs + z] : 0.0;
+  }
   double Lb[3];
   if (ND == 1) {
 #pragma unroll
@@ -700,10 +728,9 @@ __device__ __forceinline__ void update_zone(const Grid &g, const UpdateArgs &a, 
     const double FxBy0 = ct_emf(F, G, g, By, Bx, z, sx, sy), FxBym = ct_emf(F, G, g, By, Bx, z - sx, sx, sy);
     const double FyBx0 = ct_emf(G, F, g, Bx, By, z, sy, sx), FyBxm = ct_emf(G, F, g, Bx, By, z - sy, sy, sx);
     if constexpr (sizeof(T) < sizeof(double)) {   // FP32 bulk: reciprocals, zeroed fluxes dropped
-      const double idx = 1.0 / dx, idy = 1.0 / dy;
-      Lb[0] = -(FyBx0 - FyBxm) * idy;
-      Lb[1] = -(FxBy0 - FxBym) * idx;
-      Lb[2] = -(fval(F, g, Bz, z) - fval(F, g, Bz, z - sx)) * idx - (fval(G, g, Bz, z) - fval(G, g, Bz, z - sy)) * idy;
+      Lb[0] = -(FyBx0 - FyBxm) * inv.y;
+      Lb[1] = -(FxBy0 - FxBym) * inv.x;
+      Lb[2] = -(fval(F, g, Bz, z) - fval(F, g, Bz, z - sx)) * inv.x - (fval(G, g, Bz, z) - fval(G, g, Bz, z - sy)) * inv.y;
     } else {   // the reference's expressions, bit for bit
       Lb[0] = -(0.0 - 0.0) / dx - (FyBx0 - FyBxm) / dy;
       Lb[1] = -(FxBy0 - FxBym) / dx - (0.0 - 0.0) / dy;
@@ -717,10 +744,9 @@ __device__ __forceinline__ void update_zone(const Grid &g, const UpdateArgs &a, 
     const double FzBx0 = ct_emf(H, F, g, Bx, Bz, z, sz, sx), FzBxm = ct_emf(H, F, g, Bx, Bz, z - sz, sz, sx);
     const double FxBz0 = ct_emf(F, H, g, Bz, Bx, z, sx, sz), FxBzm = ct_emf(F, H, g, Bz, Bx, z - sx, sx, sz);
     if constexpr (sizeof(T) < sizeof(double)) {   // FP32 bulk: reciprocals, zeroed fluxes dropped
-      const double idx = 1.0 / dx, idy = 1.0 / dy, idz = 1.0 / dz;
-      Lb[0] = -(FyBx0 - FyBxm) * idy - (FzBx0 - FzBxm) * idz;
-      Lb[1] = -(FxBy0 - FxBym) * idx - (FzBy0 - FzBym) * idz;
-      Lb[2] = -(FxBz0 - FxBzm) * idx - (FyBz0 - FyBzm) * idy;
+      Lb[0] = -(FyBx0 - FyBxm) * inv.y - (FzBx0 - FzBxm) * inv.z;
+      Lb[1] = -(FxBy0 - FxBym) * inv.x - (FzBy0 - FzBym) * inv.z;
+      Lb[2] = -(FxBz0 - FxBzm) * inv.x - (FyBz0 - FyBzm) * inv.y;
     } else {   // the reference's expressions, bit for bit
       Lb[0] = -(0.0 - 0.0) / dx - (FyBx0 - FyBxm) / dy - (FzBx0 - FzBxm) / dz;
       Lb[1] = -(FxBy0 - FxBym) / dx - (0.0 - 0.0) / dy - (FzBy0 - FzBym) / dz;
@@ -729,14 +755,14 @@ __device__ __forceinline__ void update_zone(const Grid &g, const UpdateArgs &a, 
   }
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
-    const double un = Un.B[c * g.cs + z];
+    const double un = bn[c], us = bs[c];
     const double L = Lb[c];
     double out;
     switch (a.combine) {
     case COMB_EULER: out = un + dtd * L; break;
-    case COMB_RK2_2: out = 0.5 * (un + Us.B[c * g.cs + z] + dtd * L); break;
-    case COMB_RK3_2: out = 3. / 4 * un + 1. / 4 * Us.B[c * g.cs + z] + 1. / 4 * dtd * L; break;
-    case COMB_RK3_3: out = 1. / 3 * un + 2. / 3 * Us.B[c * g.cs + z] + 2. / 3 * dtd * L; break;
+    case COMB_RK2_2: out = 0.5 * (un + us + dtd * L); break;
+    case COMB_RK3_2: out = 3. / 4 * un + 1. / 4 * us + 1. / 4 * dtd * L; break;
+    case COMB_RK3_3: out = 1. / 3 * un + 2. / 3 * us + 2. / 3 * dtd * L; break;
     case COMB_RK4_K: { const double kk = dtd * L; Kout.B[c * g.cs + z] = kk; out = un + a.c * kk; } break;
     default:
       out = un + (1.0 / 6.0) * (K1.B[c * g.cs + z] + 2.0 * K2.B[c * g.cs + z] + 2.0 * K3.B[c * g.cs + z] + dtd * L);
@@ -746,8 +772,19 @@ __device__ __forceinline__ void update_zone(const Grid &g, const UpdateArgs &a, 
   }
 }
 
+template <class T, int ND>
+__device__ __forceinline__ void update_zone(const Grid &g, const UpdateArgs &a, StateCPtr<T> Un, StateCPtr<T> Us,
+                                            const T *__restrict__ F, const T *__restrict__ G,
+                                            const T *__restrict__ H, StatePtr<T> Uout, StatePtr<T> Kout,
+                                            StateCPtr<T> K1, StateCPtr<T> K2, StateCPtr<T> K3, double dtd,
+                                            double3 inv, long long z)
+{
+  update_bulk<T, ND>(g, a, Un, Us, F, G, H, Uout, Kout, K1, K2, K3, dtd, z);
+  update_field<T, ND>(g, a, Un, Us, F, G, H, Uout, Kout, K1, K2, K3, dtd, inv, z);
+}
+
 #ifndef MGPU_UPDATE_MINB
-#define MGPU_UPDATE_MINB 4   // 64 registers: chosen by a sweep of 3-4 (the natural count, 74, allows 3)
+#define MGPU_UPDATE_MINB 4   // 64 registers: 96^3 FP32 RK2 with 4 blocks 0.117 ms, with 3 0.126
 #endif
 
 template <class T, int ND>
@@ -755,12 +792,12 @@ __global__ void __launch_bounds__(256, MGPU_UPDATE_MINB) k_update(Grid g, Update
                                                 const T *__restrict__ F, const T *__restrict__ G,
                                                 const T *__restrict__ H, StatePtr<T> Uout, StatePtr<T> Kout,
                                                 StateCPtr<T> K1, StateCPtr<T> K2, StateCPtr<T> K3,
-                                                const Ctl *ctl, int stage)
+                                                const Ctl *ctl, int stage, double3 inv)
 {
   if (stage_failed(ctl, stage + 1)) return;
   const long long t = (long long) blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= g.ninterior) return;
-  update_zone<T, ND>(g, a, Un, Us, F, G, H, Uout, Kout, K1, K2, K3, ctl->dt, interior_zone(g, t));
+  update_zone<T, ND>(g, a, Un, Us, F, G, H, Uout, Kout, K1, K2, K3, ctl->dt, inv, interior_zone(g, t));
 }
 
 }  // namespace mgpu
