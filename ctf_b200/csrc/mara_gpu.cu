@@ -80,7 +80,7 @@ void pipe_free(mgpu_solver *h, bool streams)
   h->pipe_host_state = 0;
   if (h->xfer_host) cudaFreeHost(h->xfer_host);
   h->xfer_host = nullptr;
-  h->xfer_host_state = 0;
+  h->xfer_host_state = h->xfer_small = 0;
   if (!streams) return;
   for (cudaEvent_t e : h->pipe_ev) cudaEventDestroy(e);
   h->pipe_ev.clear();
@@ -520,16 +520,23 @@ static int transfer(mgpu_solver *h, double *host, const void *dev_in, void *dev_
     CK(cudaStreamSynchronize(h->stream));
     return MGPU_OK;
   }
-  // a pageable buffer from 4 MB on goes through two pinned chunk slots (xfer_host), chunk by chunk:
-  // the threaded host copy of one chunk overlaps the DMA copy and conversion of the other (the
-  // driver moves pageable memory at about 13 GB/s; a 64^3 FP64 Mara.advance, 22 MB each way,
-  // took 4.8 ms with the driver's copies)
+  // a pageable buffer goes through two pinned chunk slots (xfer_host), chunk by chunk: the threaded
+  // host copy of one chunk overlaps the DMA copy and conversion of the other (the driver moves
+  // pageable memory at about 13 GB/s; a 64^3 FP64 Mara.advance, 22 MB each way, took 4.8 ms with
+  // the driver's copies).  Below 64 MB making the slots costs as much as some eight transfers
+  // gain, so a solver's first eight go as they are: a solver that is filled, advanced and read
+  // once does not pay for slots that it hardly uses.
   bool staged = false;
-  if ((size_t) (nz - zbeg) * 8 * sizeof(double) >= (size_t(4) << 20)) {
+  const size_t bytes = (size_t) (nz - zbeg) * 8 * sizeof(double);
+  if (bytes >= (size_t(4) << 20)) {
     cudaPointerAttributes pa{};
     const bool pinned = cudaPointerGetAttributes(&pa, host + zbeg * 8) == cudaSuccess && pa.type == cudaMemoryTypeHost;
     cudaGetLastError();   // an unregistered pointer may leave an error behind
-    staged = !pinned && xfer_host_setup(h);
+    if (!pinned) {
+      const bool wait = bytes < (size_t(64) << 20) && h->xfer_host_state == 0 && h->xfer_small < 8;
+      if (wait) ++h->xfer_small;
+      else staged = xfer_host_setup(h);
+    }
   }
   const long long chunk = staged ? xfer_chunk(h, nz - zbeg) : h->staging_zones, slot_doubles = chunk * 8;
   auto slot = [&](int c) { return h->xfer_host + (c % 2) * slot_doubles; };

@@ -60,6 +60,7 @@ struct mgpu_solver {
   HostCopyPool *pipe_pool = nullptr;
   // the plain host transfers of a large pageable buffer: two pinned chunk slots and their events
   double *xfer_host = nullptr;
+  int xfer_small = 0;                   // transfers below 64 MB made before the slots were
   int xfer_host_state = 0;
   std::vector<cudaEvent_t> xfer_ev;
 };
