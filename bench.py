@@ -100,15 +100,16 @@ CFL = 0.3
 # utilisation that bounds the lean HLLD sweeps.  They come from separate captures, not from
 # the run that prints them.
 NCU_TRAFFIC_PER_UNIT = {("update", "plm", "hlld", "lean"): 69.7,    # a first-stage CT launch
-                        # the x sweep's DRAM bytes per zone, 120.2 against its 100 algorithmic,
-                        # applied as that 1.202 ratio to the mean of the three sweeps (86.7 B)
-                        ("flux", "plm", "hlld", "lean"): 104.2}
+                        # a first-stage x sweep's DRAM bytes per zone, 104.1 against its 80
+                        # algorithmic, applied as that 1.301 ratio to the mean of the three sweeps
+                        # (86.7 B); for WENO5 a y sweep's 82.2 against 80
+                        ("flux", "plm", "hlld", "lean"): 112.8,
+                        ("flux", "weno5", "hlld", "lean"): 89.1}
 NCU_LIMITER = {
-    ("flux", "plm", "hlld", "lean"): {"issue_active": 0.507, "fma_pipe": 0.263, "xu_pipe": 0.133,
-                                      "dram_throughput": 0.086},
-    ("flux", "weno5", "hlld", "lean"): {"issue_active": 0.467, "fma_pipe": 0.281, "xu_pipe": 0.194,
-                                        "dram_throughput": 0.068},
-    ("flux", "weno5", "hlld", "standard"): {"issue_active": 0.500, "fma_pipe": 0.292, "xu_pipe": 0.210},
+    ("flux", "plm", "hlld", "lean"): {"issue_active": 0.683, "fma_pipe": 0.382, "xu_pipe": 0.197,
+                                      "dram_throughput": 0.148},
+    ("flux", "weno5", "hlld", "lean"): {"issue_active": 0.619, "fma_pipe": 0.380, "xu_pipe": 0.244,
+                                        "dram_throughput": 0.090},
 }
 
 
@@ -918,8 +919,7 @@ def main():
     # DRAM bytes per work unit (face for the standard flux kernel, interior zone otherwise)
     # from one ncu capture of the same kernel on a 160^3 box of the same scheme -- not this
     # run -- scaled to this launch's units (lean sweeps: the mean of the x, y and z sweeps)
-    measured = {("flux", "weno5", "hlld", "standard"): 80.0, ("update", "weno5", "hlld", "standard"): 219.8,
-                ("flux", "weno5", "hlld", "lean"): 105.1}
+    measured = {("update", "weno5", "hlld", "standard"): 219.8}
     measured.update(NCU_TRAFFIC_PER_UNIT)
     tpu = measured.get((dom, scheme_kw["extrap"], scheme_kw["riemann"], args.layout)) \
         if head_key.startswith("fp32") else None
