@@ -1321,10 +1321,11 @@ static __device__ __noinline__ HlldRoot hlld_newton_cold(HlldEqn<double> q, doub
 
 // Walks p from the guess to the root of equation 48 (or, with `direct`, stays at it) and leaves
 // the states at the final pressure in f: one evaluation site for the iteration and the flux.
-// `guess` gives the reference's own starting pressure, for hlld_newton.
+// `guess` gives the reference's own starting pressure, for hlld_newton; with `weak` that runs
+// at once.
 template <class Guess>
-__device__ __forceinline__ int hlld_solve(const HlldEqn<double> &q, bool direct, double &p, HlldFill<double> &f,
-                                          const Guess &guess)
+__device__ __forceinline__ int hlld_solve(const HlldEqn<double> &q, bool direct, bool weak, double &p,
+                                          HlldFill<double> &f, const Guess &guess)
 {
   using Tol = RmhdTol<double>;
   const double dp = Tol::jac_dp;
@@ -1337,7 +1338,7 @@ __device__ __forceinline__ int hlld_solve(const HlldEqn<double> &q, bool direct,
     if (last) return 0;
     const double y = hlld_residual(f);
     // where K_R and K_L agree the residual is zero by definition, not by convergence
-    bool ok = !(fabs(f.Kr[0] - f.Kl[0]) < Tol::k_small);
+    bool ok = !weak && !(fabs(f.Kr[0] - f.Kl[0]) < Tol::k_small);
     if (it == 0) {
       y0 = y;
       p = x0 + dp;
@@ -1610,7 +1611,10 @@ __device__ __forceinline__ int riemann_hlld64(const PhysParams &pp, int dim, con
   // The HLL state and flux, and from them the first pressure guess.  The iteration converges to
   // the same root from a guess good to 1e-6, so the HLL state is inverted in FP32 where its
   // pressure and velocity are clear of the checks the reference's inversion makes; elsewhere,
-  // and for the faces that run the reference's own Newton, in FP64 (hll_guess64).
+  // and for the faces that run the reference's own Newton, in FP64 (hll_guess64).  Among those
+  // are the faces of a weak normal field, |Bx| < 1e-5 sqrt(p): the residual there is of the
+  // order of Bx (K_R - K_L), so that it passes within a step of any guess and the result would
+  // keep what the FP32 guess is off by (fluxes up to 1e-6 off at |Bx| = 1e-7).
   T U_hll[8], F_hll[3];
   {
     const Recip<T> iS = recip(ap - am);
@@ -1653,6 +1657,7 @@ __device__ __forceinline__ int riemann_hlld64(const PhysParams &pp, int dim, con
     if (tally) { tally->iters = it; tally->attempts = 1; }
     if (hll_c2p_failed) hll_c2p_failed = guess64(p_est0);
   }
+  const bool weak = q.bx * q.bx < T(1e-10) * p_est0;
   // HlldEquation48 constructor (riemann_hlld-rmhd.cpp:315-345)
   q.ap = ap;
   q.am = am;
@@ -1699,7 +1704,7 @@ __device__ __forceinline__ int riemann_hlld64(const PhysParams &pp, int dim, con
       if (est == 0) guess64(p);
       return p;
     };
-    int rc = hlld_solve(q, direct, p_star, fill, start);
+    int rc = hlld_solve(q, direct, weak, p_star, fill, start);
     if (rc == 0) rc = hlld_reconstruct(q, p_star, fill, col, F);
     success = (rc == 0);
     ++attempt;

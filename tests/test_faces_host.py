@@ -146,3 +146,16 @@ def test_relativistic_jumps_fall_back_to_hllc_where_the_oracle_does(lib, wmax):
     assert np.array_equal(u, u0), np.flatnonzero(u != u0)
     ok = e0 == 0
     assert face_rel(F[ok], F0[ok]).max() <= 1e-10   # the whole-step bound, face by face
+
+
+@pytest.mark.parametrize("wmax", [1.5, 3.0, 10.0])
+@pytest.mark.parametrize("bn", [2e-8, 1e-7, 1e-6])
+def test_weak_normal_fields_keep_the_oracle_bits(lib, wmax, bn):
+    """Equation 48's residual scales with the normal field, so that at |Bx| far below sqrt(p) it
+    passes wherever the iteration starts: only the reference's own start and iteration give
+    its flux, and they give every bit of it."""
+    P, Q = random_faces(2000, wmax, 0.05, bn)
+    F0, e0, u0 = oracle_hlld(P, Q)
+    F, e, u = host_hlld(lib, P, Q)
+    assert np.array_equal(e, e0) and np.array_equal(u, u0)
+    assert np.array_equal(F[e0 == 0], F0[e0 == 0])
