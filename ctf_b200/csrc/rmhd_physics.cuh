@@ -1299,12 +1299,16 @@ __device__ __forceinline__ int hlld_newton(const HlldEqn<T> &q, T &x)
 // at the starting pressure, then inverse interpolation through the points already there --
 // Newton's first step and about its second from three evaluations, where the central
 // differences of each Newton iteration take three -- and as in hlld_newton a last step from the
-// point whose residual passes.  Faces on which the residual does not fall twentyfold in the
-// first step and fiftyfold in the later ones (or is NaN) run hlld_newton from the start, out of
-// line, and keep the reference's outcome: eq. 48 has other roots, and without this bound one
-// face in 10^8 took one.  So do faces on which K_R and K_L meet on the way: the reference sets
-// the residual to zero there, its Newton then divides by a zero slope and rejects the attempt,
-// and the face falls back to HLLC (6% of the faces of magnetised jumps at Lorentz factor 50).
+// point whose residual passes, or a last two: the slope here is good to a few percent, so that
+// a step of 4e-12 p leaves p off by 1e-13, hlld_newton's own accuracy.
+//
+// Faces on which the residual does not fall twentyfold in the first step and fiftyfold in the
+// later ones (or is NaN) run hlld_newton from the start, out of line, and keep the reference's
+// outcome: eq. 48 has other roots, and without this bound one face in 10^8 took one.  So do
+// faces on which K_R and K_L meet on the way: the reference sets the residual to zero there, its
+// Newton then divides by a zero slope and rejects the attempt, and the face falls back to HLLC
+// (6% of the faces of magnetised jumps at Lorentz factor 50).
+//
 // Newton takes 6 to 12 evaluations on turbulence faces and this 4 or 5 (360,000 faces: fluxes
 // within 1e-14 on 99.9%, the same branch on all).
 struct HlldRoot {
@@ -1331,7 +1335,7 @@ __device__ __forceinline__ int hlld_solve(const HlldEqn<double> &q, bool direct,
   const double dp = Tol::jac_dp;
   double x0 = p, y0 = 0.0, s0 = 0.0, sl = 0.0;   // the start, its residual and dx/dy; the latest dx/dy
   double x1 = 0.0, y1 = 0.0;             // the latest point
-  bool last = direct;
+  bool last = direct, passed = false;
 #pragma unroll 1
   for (int it = 0;; ++it) {
     hlld_fill(q, p, f);
@@ -1364,7 +1368,11 @@ __device__ __forceinline__ int hlld_solve(const HlldEqn<double> &q, bool direct,
       y1 = y;
       p -= step;
     }
-    last = fabs(y1) <= Tol::newton_eps;
+    // one evaluation more where the residual passes with a step that the slope's last few percent
+    // matter in: the residual's scale is that of the normal field, and 1e-12 of it can be 1e-9 of p
+    const bool passes = fabs(y1) <= Tol::newton_eps;
+    last = passes && (passed || fabs(p - x1) <= 4e-12 * fabs(p));
+    passed = passes;
     if (!ok || !(fabs(p) < 1e300)) {
       const HlldRoot r = hlld_newton_cold(q, guess());
       if (r.err) return 1;

@@ -159,3 +159,16 @@ def test_weak_normal_fields_keep_the_oracle_bits(lib, wmax, bn):
     F, e, u = host_hlld(lib, P, Q)
     assert np.array_equal(e, e0) and np.array_equal(u, u0)
     assert np.array_equal(F[e0 == 0], F0[e0 == 0])
+
+
+@pytest.mark.parametrize("bn", [1e-3, 3e-3])
+def test_small_normal_fields_are_iterated_to_the_oracle_accuracy(lib, bn):
+    """The pressure ends within the slope's last few percent of a step of 4e-12 (2e-13), and the
+    residual's rounding (1e-16 of the Alfven speeds, whose difference is of the order of the
+    normal field) adds 1e-16 / bn (1e-13): 5e-13 allows for both and the fluxes' own rounding."""
+    P, Q = random_faces(40000, 20.0, 0.02, bn)
+    F0, e0, u0 = oracle_hlld(P, Q)
+    F, e, u = host_hlld(lib, P, Q)
+    assert np.array_equal(e, e0) and np.array_equal(u, u0)
+    ok = e0 == 0
+    assert face_rel(F[ok], F0[ok]).max() <= 5e-13
