@@ -58,6 +58,19 @@ extern "C" void hlld64(int n, const int *dim, const double *pl, const double *pr
     for (int q = 0; q < 8; ++q) F[frame_slot(dim[i], q)] = f[q];
   }
 }
+
+// the fast speeds of single states (dimension 1), as the HLL / HLLC sweeps and as the HLLD sweeps take them
+extern "C" void speeds32(int n, const float *P, float *out)
+{
+  for (int i = 0; i < n; ++i, P += 8, out += 4) {
+    float U[8], F[8];
+    prim_to_cons(4.f / 3.f, P, U);
+    flux_and_eigenvalues(4.f / 3.f, U, P, F, out[0], out[1], 1);
+    SideState s, t;
+    float ml = 0.f;
+    face_sides(4.f / 3.f, P, P, P[Bx], s, t, out[2], out[3], ml);
+  }
+}
 """
 
 _i, _d, _f = (np.ctypeslib.ndpointer(dtype=t, flags="C_CONTIGUOUS") for t in (np.int32, np.float64, np.float32))
@@ -78,6 +91,7 @@ def lib(tmp_path_factory):
     assert r.returncode == 0, r.stderr[-3000:]
     L = ctypes.CDLL(str(d / "faces.so"))
     L.hlld64.argtypes = [ctypes.c_int, _i, _d, _d, _d, _i, _i]
+    L.speeds32.argtypes = [ctypes.c_int, _f, _f]
     return L
 
 
@@ -172,3 +186,56 @@ def test_small_normal_fields_are_iterated_to_the_oracle_accuracy(lib, bn):
     assert np.array_equal(e, e0) and np.array_equal(u, u0)
     ok = e0 == 0
     assert face_rel(F[ok], F0[ok]).max() <= 5e-13
+
+
+# ---- FP32 fast speeds ---------------------------------------------------------------------------
+
+def fast_speeds(P):
+    """The extreme roots (largest, smallest) of the fast magnetosonic quartic of the states P
+    (direction 1), in extended precision:
+      rho h (1 - cs^2) W^4 d^4 = (1 - l^2) ((b^2 + rho h cs^2) W^2 d^2 - cs^2 (b^x - l b^0)^2),
+    l = v + d, in units of d / s with s^2 = cs^2 + b^2 / rho h.  From outside the roots, Newton's
+    iteration falls onto them monotonically."""
+    P = P.astype(np.longdouble)
+    rho, p, v, vB = P[:, 0], P[:, 1], P[:, 2], (P[:, 2:5] * P[:, 5:]).sum(1)
+    iW2 = 1 - (P[:, 2:5] ** 2).sum(1)
+    rh = rho + p * 4
+    cs2, b2 = GAMMA * p / rh, (P[:, 5:] ** 2).sum(1) * iW2 + vB ** 2
+    s2 = cs2 + b2 / rh
+    s = np.sqrt(s2)
+    w = P[:, 5] * iW2                       # (b^x - l b^0) / W = w - d vB
+    out = []
+    for sg in (1, -1):
+        def f(x):
+            d = s * x
+            return (1 - cs2) / iW2 * x ** 4 - (1 - (v + d) ** 2) * (x ** 2 - cs2 / rh * ((w - d * vB) / s2) ** 2)
+        x = sg * (1 + np.abs(v)) / s        # outside |l| = 1
+        x = sg * np.minimum(np.abs(x), 1 / s + 2)
+        for _ in range(400):
+            h = np.abs(x) * np.longdouble(1e-9)
+            df = (f(x + h) - f(x - h)) / (2 * h)
+            x = x - f(x) / df
+        out.append((v + s * x).astype(np.float64))
+    return out
+
+
+def cold_states():
+    rng = np.random.default_rng(3)
+    rows = []
+    for p in 10.0 ** np.arange(-36, 1, 2):
+        for v in ((0.0, 0.0, 0.0), (0.1, 0.2, 0.1), (-0.6, 0.3, 0.2)):
+            for B in ((0.3, 0.1, 0.2), (1e-3, 1e-3, 2e-3), (0.0, 0.5, 0.0), (2.0, -1.0, 0.5)):
+                rows.append((1.0, p) + v + tuple(b * rng.uniform(0.8, 1.2) for b in B))
+    return np.array(rows, dtype=np.float32)
+
+
+def test_fp32_speeds_down_to_the_coldest_gas(lib):
+    """Coefficients rounded to some 1e-7 and roots that are simple: 1e-5 allows for a condition of
+    a hundred."""
+    P = cold_states()
+    out = np.zeros((len(P), 4), np.float32)
+    lib.speeds32(len(P), P, out)
+    hi, lo = fast_speeds(P)
+    for k in (0, 2):
+        assert np.abs(out[:, k] - hi).max() <= 1e-5, (k, P[np.abs(out[:, k] - hi).argmax()])
+        assert np.abs(out[:, k + 1] - lo).max() <= 1e-5, (k, P[np.abs(out[:, k + 1] - lo).argmax()])
