@@ -80,8 +80,11 @@ __device__ __forceinline__ int side_state(float gamma, float rh_p, float r, floa
   if (near) {
     const float tol = 0.02f * (a - b);
     if (fabsf(o.bhi - near->bhi) < tol && fabsf(o.blo - near->blo) < tol) {
-      a += near->hi - near->bhi;
-      b += near->lo - near->blo;
+      const float c = a + (near->hi - near->bhi), d = b + (near->lo - near->blo);
+      if (laguerre_start(q, c, 1.f) && laguerre_start(q, d, -1.f)) {
+        a = c;
+        b = d;
+      }
     }
   }
   laguerre_pair(q, a, b);

@@ -71,6 +71,16 @@ extern "C" void speeds32(int n, const float *P, float *out)
     face_sides(4.f / 3.f, P, P, P[Bx], s, t, out[2], out[3], ml);
   }
 }
+
+// a face's outer speeds (dimension 1)
+extern "C" void face_speeds32(int n, const float *pl, const float *pr, float *out)
+{
+  for (int i = 0; i < n; ++i, pl += 8, pr += 8, out += 2) {
+    SideState s, t;
+    float ml = 0.f;
+    face_sides(4.f / 3.f, pl, pr, pl[Bx], s, t, out[0], out[1], ml);
+  }
+}
 """
 
 _i, _d, _f = (np.ctypeslib.ndpointer(dtype=t, flags="C_CONTIGUOUS") for t in (np.int32, np.float64, np.float32))
@@ -92,6 +102,7 @@ def lib(tmp_path_factory):
     L = ctypes.CDLL(str(d / "faces.so"))
     L.hlld64.argtypes = [ctypes.c_int, _i, _d, _d, _d, _i, _i]
     L.speeds32.argtypes = [ctypes.c_int, _f, _f]
+    L.face_speeds32.argtypes = [ctypes.c_int, _f, _f, _f]
     return L
 
 
@@ -211,7 +222,7 @@ def fast_speeds(P):
             return (1 - cs2) / iW2 * x ** 4 - (1 - (v + d) ** 2) * (x ** 2 - cs2 / rh * ((w - d * vB) / s2) ** 2)
         x = sg * (1 + np.abs(v)) / s        # outside |l| = 1
         x = sg * np.minimum(np.abs(x), 1 / s + 2)
-        for _ in range(400):
+        for _ in range(60):
             h = np.abs(x) * np.longdouble(1e-9)
             df = (f(x + h) - f(x - h)) / (2 * h)
             x = x - f(x) / df
@@ -239,3 +250,28 @@ def test_fp32_speeds_down_to_the_coldest_gas(lib):
     for k in (0, 2):
         assert np.abs(out[:, k] - hi).max() <= 1e-5, (k, P[np.abs(out[:, k] - hi).argmax()])
         assert np.abs(out[:, k + 1] - lo).max() <= 1e-5, (k, P[np.abs(out[:, k + 1] - lo).argmax()])
+
+
+@pytest.mark.parametrize("angle,jump,dv", [(0.01, 0.1, 0.02), (0.05, 0.02, 0.02), (0.02, 0.05, 0.01)])
+def test_fp32_outer_speeds_where_fast_and_slow_meet(lib, angle, jump, dv):
+    """Faces with the field nearly along the sweep and Alfven and sound speeds nearly equal: the
+    fast and slow roots of a side almost coincide, and the other side's correction must not
+    start its iteration between them.  Rounding of 1e-7 in the coefficients moves a double
+    root by the square root of that: 1e-3 allows for a condition of ten."""
+    rng = np.random.default_rng(11)
+    n = 4000
+    p, rho = np.exp(rng.uniform(np.log(0.1), np.log(10), n)), np.exp(0.1 * rng.standard_normal(n))
+    rh = rho + 4 * p
+    cs2 = GAMMA * p / rh
+    B = np.sqrt(rh * cs2 / (1 - cs2) * np.exp(0.1 * rng.standard_normal(n)))   # Alfven speed ~ sound speed
+    th, ph = angle * rng.random(n), 2 * np.pi * rng.random(n)
+    P = np.stack([rho, p] + [0.01 * rng.standard_normal(n) for _ in range(3)] +
+                 [B * np.cos(th), B * np.sin(th) * np.cos(ph), B * np.sin(th) * np.sin(ph)], axis=1)
+    Q = P * (1 + jump * rng.standard_normal((n, 8)) * np.array([1, 1, 0, 0, 0, 0, 1, 1]))
+    Q[:, 2:5] += dv * rng.standard_normal((n, 3))
+    P, Q = P.astype(np.float32), Q.astype(np.float32)
+    out = np.zeros((n, 2), np.float32)
+    lib.face_speeds32(n, P, Q, out)
+    l, r = fast_speeds(P), fast_speeds(Q)
+    assert np.abs(out[:, 0] - np.maximum(l[0], r[0])).max() <= 1e-3
+    assert np.abs(out[:, 1] - np.minimum(l[1], r[1])).max() <= 1e-3
