@@ -798,15 +798,36 @@ __device__ __forceinline__ T max3(T a, T b, T c)
   return x01 > c ? x01 : c;
 }
 
+// The smaller and the larger of two numbers, NaN when either is.
+#ifdef __CUDA_ARCH__
+__device__ __forceinline__ float min_nan(float a, float b)
+{
+  float r;
+  asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float max_nan(float a, float b)
+{
+  float r;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+  return r;
+}
+#else
+__device__ __forceinline__ float min_nan(float a, float b) { return isnan(a) || isnan(b) ? a + b : fminf(a, b); }
+__device__ __forceinline__ float max_nan(float a, float b) { return isnan(a) || isnan(b) ? a + b : fmaxf(a, b); }
+#endif
+
 // minmod of three slopes, as the reference's 0.25 |sgn a + sgn b| (sgn a + sgn c) min(|a|, |b|, |c|):
-// the common sign times the smallest magnitude, or zero.  In FP32 by minima and maxima (six
-// operations without the integer signs and their conversions; the same value for every
-// triple of numbers).
+// the common sign times the smallest magnitude, or zero.  In FP32 by minima and maxima: c held
+// between zero and the minmod of a and b (six operations without the integer signs and their
+// conversions; the same value for every triple of finite numbers).  A NaN c gives NaN, as there,
+// and NaN a and b (the far zone's, whose sign counts as zero) give zero.
 template <class T>
 __device__ __forceinline__ T minmod3(T a, T b, T c)
 {
   if constexpr (sizeof(T) < sizeof(double)) {
-    return fmaxf(fminf(fminf(a, b), c), 0.f) + fminf(fmaxf(fmaxf(a, b), c), 0.f);
+    const float hi = fmaxf(fminf(a, b), 0.f), lo = fminf(fmaxf(a, b), 0.f);
+    return min_nan(max_nan(c, lo), hi);
   } else {
     const int sa = sgn(a), sb = sgn(b), sc = sgn(c);
     return T(0.25) * T(abs(sa + sb)) * T(sa + sc) * min3(m_abs(a), m_abs(b), m_abs(c));

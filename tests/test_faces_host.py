@@ -72,6 +72,15 @@ extern "C" void speeds32(int n, const float *P, float *out)
   }
 }
 
+// minmod of slope triples: 32 the FP32 form, 64 the reference's expression
+extern "C" void minmod(int n, const float *abc, float *f32, double *f64)
+{
+  for (int i = 0; i < n; ++i, abc += 3) {
+    f32[i] = minmod3(abc[0], abc[1], abc[2]);
+    f64[i] = minmod3(double(abc[0]), double(abc[1]), double(abc[2]));
+  }
+}
+
 // a face's outer speeds (dimension 1)
 extern "C" void face_speeds32(int n, const float *pl, const float *pr, float *out)
 {
@@ -102,6 +111,7 @@ def lib(tmp_path_factory):
     L = ctypes.CDLL(str(d / "faces.so"))
     L.hlld64.argtypes = [ctypes.c_int, _i, _d, _d, _d, _i, _i]
     L.speeds32.argtypes = [ctypes.c_int, _f, _f]
+    L.minmod.argtypes = [ctypes.c_int, _f, _f, _d]
     L.face_speeds32.argtypes = [ctypes.c_int, _f, _f, _f]
     return L
 
@@ -275,3 +285,13 @@ def test_fp32_outer_speeds_where_fast_and_slow_meet(lib, angle, jump, dv):
     l, r = fast_speeds(P), fast_speeds(Q)
     assert np.abs(out[:, 0] - np.maximum(l[0], r[0])).max() <= 1e-3
     assert np.abs(out[:, 1] - np.minimum(l[1], r[1])).max() <= 1e-3
+
+
+def test_fp32_minmod_is_the_reference_expression(lib):
+    """PLM slopes of three zones, any of which may be NaN."""
+    rng = np.random.default_rng(5)
+    v = rng.choice(np.array([-2.0, -1.0, -0.5, 0.0, 0.25, 1.0, 3.0, np.nan], np.float32), (20000, 3))
+    abc = np.stack([2 * (v[:, 1] - v[:, 0]), 0.5 * (v[:, 2] - v[:, 0]), 2 * (v[:, 2] - v[:, 1])], axis=1)
+    f32, f64 = np.zeros(len(v), np.float32), np.zeros(len(v))
+    lib.minmod(len(v), np.ascontiguousarray(abc, dtype=np.float32), f32, f64)
+    assert np.isnan(f64).any() and np.array_equal(f32, f64.astype(np.float32), equal_nan=True)
