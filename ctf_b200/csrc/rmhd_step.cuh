@@ -89,7 +89,7 @@ __device__ __forceinline__ void stat_reset(Ctl *ctl)
     reinterpret_cast<unsigned long long *>(ctl->stat)[i] = 0ull;
 }
 
-// Warp-aggregated counter increment.
+// Warp-aggregated counter increment: every active lane must pass the same counter.
 __device__ __forceinline__ void warp_add(unsigned long long *ctr, unsigned v)
 {
   const unsigned mask = __activemask();
@@ -186,7 +186,11 @@ __device__ __forceinline__ void c2p_finish(const Grid &g, T *PA, StatePtr<T> Pn,
     StatSlot &st = stat_slot(ctl);
     warp_add(&st.c2p_calls, 1u);
     warp_add(&st.c2p_iters, (unsigned) tally.iters);
-    if (tally.attempts != 1) warp_add(&st.c2p_attempt[tally.attempts], 1u);   // [1] is the rest
+    if (tally.attempts != 1) {   // [1] is the rest
+#pragma unroll 1
+      for (int a = 0; a < 6; ++a)   // one counter at a time: warp_add sums over the active lanes
+        if (tally.attempts == a) warp_add(&st.c2p_attempt[a], 1u);
+    }
     if (err) warp_add(&st.c2p_failed, 1u);
   }
   if (err) {
