@@ -226,6 +226,7 @@ __global__ void __launch_bounds__(128, flux_minb<RS>()) k_lean_sweep(Grid g, con
 #pragma unroll
       for (int q = 0; q < 8; ++q) up[q][threadIdx.x] = hi[q];
       solve_face<T, RS, true>(g, PA, pp, dim, f, Pl, Pr, ml, ft, Ff, cols + threadIdx.x);
+      if (m < m0 && chunk > 0) ft = FluxTally{0, 0, 0, 0, 0};   // its neighbour's last face: counted there
 #pragma unroll
       for (int q = 0; q < 8; ++q) Fo[face_slot<T, RS>(dim, q)] = Ff[q];
       if (m >= m0 || chunk == 0) {            // the chunk's first face is its neighbour's last
@@ -292,6 +293,7 @@ __global__ void __launch_bounds__(128, flux_minb<RS>()) k_lean_sweep_z(Grid g, c
 #pragma unroll
     for (int r = 0; r < 8; ++r) Pl[r] = up[r][threadIdx.x - 1];
     solve_face<T, RS, true>(g, PA, pp, 3, z - 1, Pl, Pr, ml, ft, Ff, cols + threadIdx.x);
+    if (threadIdx.x == 1 && blockIdx.x > 0) ft = FluxTally{0, 0, 0, 0, 0};   // the previous CTA's last face
 #pragma unroll
     for (int r = 0; r < 8; ++r) Fo[face_slot<T, RS>(3, r)] = Ff[r];
     if (threadIdx.x > 1 || blockIdx.x == 0) {

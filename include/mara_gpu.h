@@ -81,7 +81,9 @@ typedef struct {
   unsigned long long c2p_calls, c2p_iters;          /* zone c2p calls and Newton iterations */
   unsigned long long c2p_attempt[6];                /* attempts used: [1..4] ladder rung,
                                                        [5] learned guess rejected */
-  unsigned long long face_c2p_calls, face_c2p_iters; /* HLL-state c2p inside HLLD */
+  unsigned long long face_c2p_calls, face_c2p_iters; /* HLL-state c2p inside HLLD; its iterations
+                                                        are FP32 ones except where the FP64
+                                                        ladder had to follow */
   unsigned long long hlld_ok, hlld_hllc, pcm_retry;  /* HLLD successes / HLLC fallbacks /
                                                         PCM retries of a face */
   unsigned long long c2p_failed;                     /* zone c2p calls that failed every rung of the

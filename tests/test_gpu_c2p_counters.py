@@ -1,5 +1,5 @@
-"""The c2p outcome counters of an advance, on a box whose neighbouring zones -- lanes of one warp
--- resolve on different rungs of the ladder, against the C restatement zone by zone."""
+"""The counters of an advance: the c2p outcomes on a box whose neighbouring zones -- lanes of one warp
+-- resolve on different rungs of the ladder, against the C restatement zone by zone, and the faces of the lean sweeps, each counted once."""
 import numpy as np
 import pytest
 
@@ -55,3 +55,16 @@ def test_outcomes_of_a_warp_are_counted_each_on_its_own_rung(golden):
     st = s.stats()
     assert st["c2p_calls"] == 2 * 512 and st["c2p_failed"] == 2 * bad.sum()
     assert list(st["c2p_attempt"]) == want
+
+
+@pytest.mark.parametrize("precision,extrap", [("fp32", "plm"), ("fp32", "weno5"), ("fp64", "plm")])
+@pytest.mark.parametrize("n", [(9, 17, 33), (47, 12, 130), (20, 64, 5)])
+def test_lean_sweeps_count_each_face_once(n, precision, extrap):
+    """A chunk of a marching sweep, and a block of the z sweep, solves its first face again; short
+    chunks repeat up to one face in three."""
+    s = Solver(Scheme(precision=precision, layout="lean", extrap=extrap, advance="rk2"), n)
+    s.upload(ics.turbulence_box(n, seed=2))
+    assert s.advance(1e-4) == 0
+    st = s.stats()
+    faces = sum((n[d] + 1) * (n[(d + 1) % 3] + 2) * (n[(d + 2) % 3] + 2) for d in range(3))
+    assert st["hlld_ok"] + st["hlld_hllc"] == 2 * faces
