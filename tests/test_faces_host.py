@@ -72,6 +72,23 @@ extern "C" void speeds32(int n, const float *P, float *out)
   }
 }
 
+// the first rung of the zone c2p, as the FP64 path (accurate) and as the FP32-bulk path (fast) runs it
+extern "C" void c2p(int n, const double *U, double *accurate, double *fast, int *err)
+{
+  for (int i = 0; i < n; ++i, U += 8, accurate += 8, fast += 8) {
+    C2PState s;
+    s.gamma = 4.0 / 3.0;
+    s.gamf = 0.25;
+    s.pfloor = -1.0;
+    c2p_new_state(s, U);
+    double Z, W;
+    int it;
+    c2p_estimate(s, Z, W);
+    err[2 * i] = c2p_anton2dzw(s, Z, W, accurate, it);
+    err[2 * i + 1] = c2p_anton2dzw_fast(s, Z, W, fast, it);
+  }
+}
+
 // minmod of slope triples: 32 the FP32 form, 64 the reference's expression
 extern "C" void minmod(int n, const float *abc, float *f32, double *f64)
 {
@@ -111,6 +128,7 @@ def lib(tmp_path_factory):
     L = ctypes.CDLL(str(d / "faces.so"))
     L.hlld64.argtypes = [ctypes.c_int, _i, _d, _d, _d, _i, _i]
     L.speeds32.argtypes = [ctypes.c_int, _f, _f]
+    L.c2p.argtypes = [ctypes.c_int, _d, _d, _d, _i]
     L.minmod.argtypes = [ctypes.c_int, _f, _f, _d]
     L.face_speeds32.argtypes = [ctypes.c_int, _f, _f, _f]
     return L
@@ -295,3 +313,23 @@ def test_fp32_minmod_is_the_reference_expression(lib):
     f32, f64 = np.zeros(len(v), np.float32), np.zeros(len(v))
     lib.minmod(len(v), np.ascontiguousarray(abc, dtype=np.float32), f32, f64)
     assert np.isnan(f64).any() and np.array_equal(f32, f64.astype(np.float32), equal_nan=True)
+
+
+# ---- the FP32-bulk c2p --------------------------------------------------------------------------
+
+@pytest.mark.parametrize("wmax,plo,phi", [(1.5, 0.1, 10.0), (3.0, 0.1, 10.0), (3.0, 1e-3, 1e-2)])
+def test_fp32_bulk_c2p_ends_at_fp64_accuracy(lib, wmax, plo, phi):
+    """Both iterations end on a step below 1e-12, with an error of that step's square and the
+    rounding of the conserved state, some 1e-15 of Z = rho h W^2, which p inherits: ten times
+    that.  Where the first rung fails it fails for both."""
+    rng = np.random.default_rng(4)
+    P, _ = random_faces(4000, wmax, 0.0)
+    P[:, 1] = P[:, 0] * np.exp(rng.uniform(np.log(plo), np.log(phi), len(P)))
+    port = PortOracle(Scheme(n=(4, 4, 4)))
+    U = np.array([port.prim_to_cons(p)[0] for p in P])
+    A, B, e = np.zeros_like(U), np.zeros_like(U), np.zeros(2 * len(U), np.int32)
+    lib.c2p(len(U), U, A, B, e)
+    ok = e[::2] == 0
+    assert np.array_equal(e[::2], e[1::2]) and ok.mean() > 0.97
+    Z = (P[:, 0] + 4 * P[:, 1]) / (1 - (P[:, 2:5] ** 2).sum(1))
+    assert (np.abs(A[:, 1] - B[:, 1]) / Z)[ok].max() <= 1e-14
