@@ -123,6 +123,7 @@ def make_ic(kind, n, seed=0):
 
 
 def launches_per_step(nd, rk):
+    """At most so many launches per step, over the layouts (it sizes the profiler)."""
     ns = {"single": 1, "rk2": 2, "rk3": 3, "rk4": 4}[rk]
     return 2 + ns * (2 + nd) + 2
 
@@ -633,9 +634,10 @@ def run_decomposed_bench(args, rank, world, local):
         ms = float(t.item())
     zones = int(np.prod(n))
     nst = {"single": 1, "rk2": 2, "rk3": 3, "rk4": 4}[scheme_kw["advance"]]
-    # per advance: begin + per stage (shell c2p, core c2p, 3 sweeps, update) + closing c2p +
-    # commit, plus 4 slab pack/unpack kernels per split dimension and stage
-    per_adv = 2 + nst * (2 + 3 + 1) + 1 + nst * 4 * len(L.split())
+    # per advance: begin + per stage (shell c2p, core c2p, one launch for the sweeps of all
+    # directions, update) + closing c2p + commit, plus 4 slab pack/unpack kernels per split
+    # dimension and stage
+    per_adv = 2 + nst * (2 + 1 + 1) + 1 + nst * 4 * len(L.split())
     out = {"metric": METRIC, "value": zones * args.steps / (ms * 1e-3), "unit": UNIT, "n_gpus": world,
            "steps": args.steps, "warmup": args.warmup, "ms_per_step": ms / args.steps, "higher_is_better": True,
            "scaling": "strong", "vs_baseline": None, "dtype": "f32", "data": "synthetic",

@@ -38,6 +38,37 @@ def test_a_shifted_box_advances_to_the_shifted_result(n, layout, precision):
         assert np.array_equal(np.roll(out[0], shift, axis=(0, 1, 2)), out[1]), (extrap, riemann)
 
 
+def smooth_box(n, seed):
+    """Turbulence on a density and pressure that vary by factors of order one over the box: every
+    component's reconstruction is resolved, and none is trivial."""
+    P = ics.turbulence_box(n, seed=seed, vrms=0.3)
+    inner = P[3:-3, 3:-3, 3:-3]
+    x, y, z = np.meshgrid(*[(np.arange(m) + 0.5) / m * 2 * np.pi for m in n], indexing="ij")
+    inner[..., 0] = np.exp(0.3 * np.sin(x + 2 * y) + 0.2 * np.cos(z))
+    inner[..., 1] = np.exp(0.3 * np.cos(2 * x - z) + 0.2 * np.sin(y))
+    return ics.with_guards(np.ascontiguousarray(inner))
+
+
+@pytest.mark.parametrize("IS", ["js96", "b08", "sz10"])
+@pytest.mark.parametrize("layout", ["lean", "standard"])
+def test_fp32_weno_indicators_match_the_oracle_in_every_component(IS, layout):
+    """One step with another indicator differs by 6e-4 or more in every component; FP32 is held to
+    a twelfth of that."""
+    n, tol = (10, 9, 8), 5e-5
+    P0, out = smooth_box(n, 9), {}
+    for mode in ("js96", "b08", "sz10"):
+        kw = dict(extrap="weno5", IS=mode, riemann="hlld", advance="single")
+        cpu, out[mode] = PortOracle(OScheme(n=n, **kw)), P0.copy()
+        assert cpu.advance(out[mode], 0.02) == 0
+    s = Solver(Scheme(precision="fp32", layout=layout, extrap="weno5", IS=IS, riemann="hlld", advance="single"), n)
+    s.upload(P0.copy())
+    assert s.advance(0.02) == 0
+    P = s.download()
+    assert rel_errors(P, out[IS], 3)[0].max() <= tol
+    for mode in out:
+        assert mode == IS or rel_errors(P, out[mode], 3)[0].min() > 5 * tol, mode
+
+
 @pytest.mark.parametrize("IS", ["js96", "b08", "sz10"])
 @pytest.mark.parametrize("riemann", ["hll", "hllc", "hlld"])
 def test_fp32_weno_indicators_match_the_oracle(IS, riemann):
@@ -70,3 +101,19 @@ def test_fp32_speeds_of_hot_fast_and_field_free_states():
         # FP32 states carry 6e-8; the slowest-varying speed of these states amplifies it a
         # thousandfold at the fast = Alfven degeneracy
         assert abs(ml["fp32"] - ml["fp64"]) <= 1e-4, (v, B, p, ml)
+
+
+@pytest.mark.parametrize("riemann", ["hll", "hllc", "hlld"])
+@pytest.mark.parametrize("layout", ["lean", "standard"])
+def test_fp32_speeds_of_unequal_sides(riemann, layout):
+    """MaxLambda of a step on boxes whose faces have two different states, close (where one side's
+    speeds help to start the other's) and far apart, against the restatement."""
+    n = (12, 10, 11)
+    for P0 in (smooth_box(n, 4), box(n, 4)):
+        kw = dict(extrap="plm", riemann=riemann, advance="single")
+        cpu, Pc = PortOracle(OScheme(n=n, **kw)), P0.copy()
+        assert cpu.advance(Pc, 1e-3) == 0
+        s = Solver(Scheme(precision="fp32", layout=layout, **kw), n)
+        s.upload(P0.copy())
+        assert s.advance(1e-3) == 0
+        assert abs(s.max_lambda - cpu.max_lambda) <= 1e-4   # as in the test above

@@ -18,7 +18,9 @@ PROGRAM = r"""
 
 int main()
 {
-  const size_t sizes[] = {0, 1, 4095, size_t(8) << 20, (size_t(8) << 20) + 1, (size_t(64) << 20) + 12345,
+  // one thread copies below 1 MB; 2 MB is the small transfers' chunk
+  const size_t sizes[] = {0, 1, 4095, (size_t(1) << 20) - 1, size_t(1) << 20, (size_t(1) << 20) + 1, size_t(2) << 20,
+                          size_t(8) << 20, (size_t(8) << 20) + 1, (size_t(64) << 20) + 12345,
                           size_t(200) << 20};
   const int threads[] = {1, 3, 8};
   unsigned seed = 12345;
