@@ -584,8 +584,9 @@ __device__ __forceinline__ int c2p_newton32(float D, float E, float S2, float B2
 // the reference's bit pattern.  The start is first brought to FP32 accuracy by the same
 // iteration in FP32 (five iterations from the estimate, at a quarter of their FP64 cost).  The
 // FP64 iteration keeps the reference's bound of 1e-12 on its last step: to end it on a first
-// step below 1e-6 costs a quarter less but leaves up to 1e-9 of p at Lorentz factor 3, as a
-// step's error is its square times the state's condition.
+// step below 1e-6 costs a tenth less (160^3 lean, RK3: 0.56 against 0.62 ms per step) but leaves
+// up to 3e-10 of p at Lorentz factor 3 and p/rho 1e-3, as a step's error is its square times the
+// state's condition.
 __device__ __forceinline__ int c2p_anton2dzw_fast(const C2PState &s, double Z, double W, double *P, int &iters)
 {
   const double D = s.D, B2 = s.B2, BS2 = s.BS2, S2 = s.S2, gamf = s.gamf, Tau = s.Tau;
