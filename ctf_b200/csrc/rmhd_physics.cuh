@@ -234,13 +234,12 @@ __device__ __forceinline__ void quartic_extreme_roots(T d4, T d3, T d2, T d1, T 
 }
 
 // ---- fast magnetosonic speeds, FP32 --------------------------------------------------------------
-// The quartic of Mara/rmhd.cpp:275-305 divided by (rho h + b^2 / cs^2) W^2 and written in
-// d = lambda - v:
+// The quartic of Mara/rmhd.cpp:275-305 divided by rho h W^2 and written in d = lambda - v:
 //   c4 d^4 + c3 d^3 + c2 d^2 + c1 d + c0.
 // In this form nothing cancels (the expanded coefficients lose all their digits near
-// degenerate roots and at high W, where FP32 Ferrari left errors of order one in the speed), and
-// with c2 of order one and the roots of order sqrt(c4) / c4 no product below leaves the FP32
-// range down to p / (rho h) = 1e-35 (divided by rho h W^2 alone, c4^2 left it at 1e-19).
+// degenerate roots and at high W, where FP32 Ferrari left errors of order one in the speed).
+// A power of two then brings c2 to order one, so that no product below leaves the FP32 range
+// down to p / (rho h) = 1e-34 (without it c4^2 left it at 1e-19); it changes no bit of the roots.
 // hi, lo: the speeds at zero normal field, outside the fast roots.
 struct FastQuartic {
   float c4, c3, c2, c1, c0, hi, lo;
@@ -250,20 +249,21 @@ __device__ __forceinline__ FastQuartic fast_quartic(float gamma, float p, float 
                                                     float v, float vB, float B1)
 {
   FastQuartic q;
-  const float irh = 1.f / rh, cs2 = gamma * p * irh;
-  const float iL = 1.f / (cs2 + b2 * irh);
-  const float M = W2 * (1.f - cs2) * iL, k = cs2 * irh * iL;
+  const float irh = 1.f / rh, ics2 = rh / (gamma * p);
+  const float L0 = 1.f + b2 * irh * ics2;
+  const float s = __int_as_float(0x7f000000 - (__float_as_int(L0) & 0x7f800000));   // 2^-exponent of L0
+  const float M = W2 * (ics2 - 1.f) * s, L = L0 * s, k = irh * s;
   const float w = B1 * iW2;
   const float uu = vB * vB * k, uw = vB * w * k, ww = w * w * k;
   const float g0 = 1.f - v * v;
-  q.c4 = M + 1.f - uu;
-  q.c3 = 2.f * (v * (1.f - uu) + uw);
-  q.c2 = g0 * (uu - 1.f) + 4.f * v * uw - ww;
+  q.c4 = M + L - uu;
+  q.c3 = 2.f * (v * (L - uu) + uw);
+  q.c2 = g0 * (uu - L) + 4.f * v * uw - ww;
   q.c1 = -2.f * (v * ww + uw * g0);
   q.c0 = ww * g0;
-  const float r = sqrtf(1.f + M * g0), is = 1.f / (M + 1.f);
-  q.hi = (r - v) * is;
-  q.lo = (-r - v) * is;
+  const float r = sqrtf(L * (L + M * g0)), is = 1.f / (M + L);
+  q.hi = (r - L * v) * is;
+  q.lo = (-r - L * v) * is;
   return q;
 }
 

@@ -19,6 +19,7 @@ GAMMA = 4.0 / 3.0
 
 PROGRAM = r"""
 #include <cmath>
+#include <cstring>
 #include <cuda_runtime.h>
 #undef __noinline__
 #define __noinline__ __attribute__((noinline))
@@ -30,6 +31,8 @@ static inline float __fdividef(float a, float b)   // CUDA's delivers 0 above 2^
 {
   return fabsf(b) > 8.507059e37f ? 0.f * a : a / b;
 }
+static inline int __float_as_int(float x) { int i; memcpy(&i, &x, 4); return i; }
+static inline float __int_as_float(int i) { float x; memcpy(&x, &i, 4); return x; }
 #include "rmhd_face32.cuh"
 namespace mgpu { bool c2p_learned_guess(const void *, const C2PState &, double &, double &) { return false; } }
 using namespace mgpu;
