@@ -454,8 +454,9 @@ int mgpu_num_zones(const mgpu_solver *h, long long *nz)
 static bool pipe_host_setup(mgpu_solver *h);
 
 // Zones of a chunk of a staged host transfer of `zones` zones, so that the host copy of one chunk
-// overlaps the DMA copy of the previous one: 2 MB up to 64 MB (pinning the two slots costs a
-// solver's first transfer about 2 ms per MB), then a quarter of the array up to 64 MB.
+// overlaps the DMA copy of the previous one: 2 MB up to 64 MB, then a quarter of the array up to
+// 64 MB.  Pinning the two slots costs the transfer that makes them 3 to 5 ms at 2 MB each and
+// some 0.5 ms per MB for large ones (measured from 4 MB, 3.5 ms, to 256 MB, 105 ms).
 static long long xfer_chunk(const mgpu_solver *h, long long zones)
 {
   const long long most = std::min<long long>(h->staging_zones, 1ll << 20);
@@ -521,14 +522,16 @@ static int transfer(mgpu_solver *h, double *host, const void *dev_in, void *dev_
     return MGPU_OK;
   }
   // a pageable buffer goes through two pinned chunk slots (xfer_host), chunk by chunk: the threaded
-  // host copy of one chunk overlaps the DMA copy and conversion of the other (the driver moves
-  // pageable memory at about 13 GB/s; a 64^3 FP64 Mara.advance, 22 MB each way, took 4.8 ms with
-  // the driver's copies).  Below 64 MB making the slots costs as much as some eight transfers
-  // gain, so a solver's first eight go as they are: a solver that is filled, advanced and read
-  // once does not pay for slots that it hardly uses.
+  // host copy of one chunk overlaps the DMA copy and conversion of the other.  The driver moves
+  // pageable memory at 13 to 20 GB/s; upload / download, as they are against staged: 8 MB
+  // 0.52 / 0.57 -> 0.36 / 0.34 ms, 22 MB 1.31 / 1.48 -> 1.11 / 1.06, 64 MB 4.4 / 5.1 -> 2.5 / 2.3;
+  // 4 to 6 MB 0.30 to 0.42 -> 0.2 to 0.6, so those go as they are.  Below 64 MB making the slots
+  // costs as much as some eight transfers of 22 MB gain (25 of 8 MB, two of 64 MB), so a solver's
+  // first eight go as they are: a solver that is filled, advanced and read once does not pay for
+  // slots that it hardly uses.
   bool staged = false;
   const size_t bytes = (size_t) (nz - zbeg) * 8 * sizeof(double);
-  if (bytes >= (size_t(4) << 20)) {
+  if (bytes >= (size_t(8) << 20)) {
     cudaPointerAttributes pa{};
     const bool pinned = cudaPointerGetAttributes(&pa, host + zbeg * 8) == cudaSuccess && pa.type == cudaMemoryTypeHost;
     cudaGetLastError();   // an unregistered pointer may leave an error behind

@@ -259,7 +259,7 @@ __global__ void __launch_bounds__(128, flux_minb<RS>()) k_lean_sweep_z(Grid g, c
   const unsigned nr = g.n[2] + 2, nj = g.n[1] + 2;
   // the window's x rows and the halo rows it computes: a - 1 in [win_flo, win_fhi)
   const int alo = win_lo(g), ahi = win_hi(g), a0 = win_flo(g) + 1;
-  const unsigned total = (unsigned) (win_fhi(g) - win_flo(g)) * nj * nr;   // < 2^31: the grid is 1-D
+  const unsigned total = (unsigned) (win_fhi(g) - win_flo(g)) * nj * nr;   // < 2^31: as many zones fill no card
   const int q = (int) (blockIdx.x * 126u) - 2 + (int) threadIdx.x;
   T ml = T(0);
   FluxTally ft{0, 0, 0, 0, 0};
