@@ -13,6 +13,14 @@ GOLDEN = os.path.join(ROOT, "tests", "golden")
 def pytest_configure(config):
     config.addinivalue_line("markers", "gpu: needs a CUDA device (B200, sm_100a)")
     config.addinivalue_line("markers", "slow: longer CPU runs")
+    config.addinivalue_line("markers", "reference: needs the compiled reference (oracle/_ref, built from its sources)")
+
+
+def pytest_runtest_setup(item):
+    if item.get_closest_marker("reference"):
+        from oracle import REF_SO
+        if not os.path.exists(REF_SO):
+            pytest.skip("the compiled reference (oracle/_ref) is not built")
 
 
 @pytest.fixture(scope="session")

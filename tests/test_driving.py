@@ -23,6 +23,7 @@ def _reference_field(tmp_path, nd, P0, zeta, k1, seed, dts):
     return open(f"{tmp_path}/A.bin", "rb").read(), open(f"{tmp_path}/B.bin", "rb").read()
 
 
+@pytest.mark.reference
 @pytest.mark.parametrize("nd,P0,zeta,k1,seed", [(3, 0.01, 1.0, 3, 12345), (3, 0.2, 0.3, 2, 7), (2, 0.05, 0.5, 3, 99)])
 def test_field_and_ou_steps_match_the_reference_bytes(tmp_path, nd, P0, zeta, k1, seed):
     dts = [0.01, 0.02, 0.005]

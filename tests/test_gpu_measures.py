@@ -83,6 +83,7 @@ def test_measures_of_reference_states(golden, k):
     _check_measures(_gpu_measures(s), {nm: g[f"c{k}_{nm}"] for nm in NAMES}, Q, len(n))
 
 
+@pytest.mark.reference
 def test_measures_read_the_last_stage_primitives():
     """After an advance the measures read the last RK stage's primitives, on both sides."""
     from ctf_b200 import ics
@@ -152,6 +153,7 @@ def test_diffuse_without_failures_is_a_round_trip():
     assert np.abs(R - Q).max() <= 1e-12 * np.abs(Q).max()
 
 
+@pytest.mark.reference
 def test_scheme_change_in_place_keeps_state_and_max_lambda():
     """set_riemann / set_advance / config_solver between advances, as the reference's crash
     ladders do: the solver continues from its state and MaxLambda (get_timestep after the

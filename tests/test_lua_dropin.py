@@ -40,6 +40,7 @@ Mara.close()
 """
 
 
+@pytest.mark.reference
 def test_driver_script_runs_in_the_reference(tmp_path):
     """The driver script itself, in the reference's interpreter (CPU)."""
     n = (8, 6, 6)
@@ -255,6 +256,7 @@ def _compare_measures(lg, lr, rel):
     assert (np.abs(a - b) <= rel * scale).all(), np.abs(a - b) / scale
 
 
+@pytest.mark.reference
 def test_crash_ladder_runs_in_the_reference(tmp_path):
     """The ladder script itself in the reference's interpreter: step 3 fails and is recovered
     by diffusion plus the CTU-Hancock fallback."""
