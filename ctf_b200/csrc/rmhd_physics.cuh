@@ -1361,10 +1361,10 @@ static __device__ __noinline__ HlldRoot hlld_newton_cold(HlldEqn<double> q, doub
 
 // Walks p from the guess to the root of equation 48 (or, with `direct`, stays at it) and leaves
 // the states at the final pressure in f: one evaluation site for the iteration and the flux.
-// `guess` gives the reference's own starting pressure, for hlld_newton; with `weak` that runs
+// `guess` gives the reference's own starting pressure, for hlld_newton; with `own` that runs
 // at once.
 template <class Guess>
-__device__ __forceinline__ int hlld_solve(const HlldEqn<double> &q, bool direct, bool weak, double &p,
+__device__ __forceinline__ int hlld_solve(const HlldEqn<double> &q, bool direct, bool own, double &p,
                                           HlldFill<double> &f, const Guess &guess)
 {
   using Tol = RmhdTol<double>;
@@ -1378,7 +1378,7 @@ __device__ __forceinline__ int hlld_solve(const HlldEqn<double> &q, bool direct,
     if (last) return 0;
     const double y = hlld_residual(f);
     // where K_R and K_L agree the residual is zero by definition, not by convergence
-    bool ok = !weak && !(fabs(f.Kr[0] - f.Kl[0]) < Tol::k_small);
+    bool ok = !own && !(fabs(f.Kr[0] - f.Kl[0]) < Tol::k_small);
     if (it == 0) {
       y0 = y;
       p = x0 + dp;
@@ -1658,7 +1658,10 @@ __device__ __forceinline__ int riemann_hlld64(const PhysParams &pp, int dim, con
   // and for the faces that run the reference's own Newton, in FP64 (hll_guess64).  Among those
   // are the faces of a weak normal field, |Bx| < 1e-5 sqrt(p): the residual there is of the
   // order of Bx (K_R - K_L), so that it passes within a step of any guess and the result would
-  // keep what the FP32 guess is off by (fluxes up to 1e-6 off at |Bx| = 1e-7).
+  // keep what the FP32 guess is off by (fluxes up to 1e-6 off at |Bx| = 1e-7).  So are those of a
+  // total pressure above 1e4 or below 1e-5: the reference's difference step is an absolute 1e-8,
+  // whose slope is rounding up there and not local down here, and whether the iteration passes
+  // depends on its every step.
   T U_hll[8], F_hll[3];
   {
     const Recip<T> iS = recip(ap - am);
@@ -1701,7 +1704,7 @@ __device__ __forceinline__ int riemann_hlld64(const PhysParams &pp, int dim, con
     if (tally) { tally->iters = it; tally->attempts = 1; }
     if (hll_c2p_failed) hll_c2p_failed = guess64(p_est0);
   }
-  const bool weak = q.bx * q.bx < T(1e-10) * p_est0;
+  const bool own = q.bx * q.bx < T(1e-10) * p_est0 || !(p_est0 > T(1e-5) && p_est0 < T(1e4));
   // HlldEquation48 constructor (riemann_hlld-rmhd.cpp:315-345)
   q.ap = ap;
   q.am = am;
@@ -1748,7 +1751,7 @@ __device__ __forceinline__ int riemann_hlld64(const PhysParams &pp, int dim, con
       if (est == 0) guess64(p);
       return p;
     };
-    int rc = hlld_solve(q, direct, weak, p_star, fill, start);
+    int rc = hlld_solve(q, direct, own, p_star, fill, start);
     if (rc == 0) rc = hlld_reconstruct(q, p_star, fill, col, F);
     success = (rc == 0);
     ++attempt;

@@ -217,6 +217,21 @@ def test_weak_normal_fields_keep_the_oracle_bits(lib, wmax, bn):
     assert np.array_equal(F[e0 == 0], F0[e0 == 0])
 
 
+@pytest.mark.parametrize("scale", [1e-10, 1e-9, 1e-8, 1e-7, 1e-6, 1e-4, 1e-2, 1e2, 1e4, 1e5, 1e6, 1e7, 1e8])
+def test_pressures_far_from_one_fall_back_to_hllc_where_the_oracle_does(lib, scale):
+    """The reference's difference step is an absolute 1e-8: at pressures far above one its slopes
+    are rounding, far below one they are not local, and its own iteration alone tells which
+    faces it rejects."""
+    P, Q = random_faces(5000, 2.0, 0.3)
+    for X in (P, Q):
+        X[:, :2] *= scale
+        X[:, 5:] *= np.sqrt(scale)
+    F0, e0, u0 = oracle_hlld(P, Q)
+    F, e, u = host_hlld(lib, P, Q)
+    assert np.array_equal(e, e0) and np.array_equal(u, u0)
+    assert face_rel(F, F0)[e0 == 0].max() <= 1e-10
+
+
 @pytest.mark.parametrize("bn", [1e-3, 3e-3])
 def test_small_normal_fields_are_iterated_to_the_oracle_accuracy(lib, bn):
     """The pressure ends within the slope's last few percent of a step of 4e-12 (2e-13), and the
