@@ -280,22 +280,8 @@ __device__ __forceinline__ float laguerre_step(const FastQuartic &q, float d, fl
   return 4.f * f / (f1 + sg * sqrtf(D));
 }
 
-// Whether d lies beyond the quartic's last turning point on side sg: from there laguerre_step falls
-// onto the extreme root, from further inside it may run to the next one.  (Real roots: past its
-// vertex f'' is positive only beyond the last inflection, and there f' only beyond the turning
-// point.)
-__device__ __forceinline__ bool laguerre_start(const FastQuartic &q, float d, float sg)
-{
-  float f = q.c4, f1 = q.c4, f2 = q.c4;
-  f = f * d + q.c3; f1 = f1 * d + f; f2 = f2 * d + f1;
-  const float f3 = q.c4 * d + f2;
-  f = f * d + q.c2; f1 = f1 * d + f; f2 = f2 * d + f1;
-  f = f * d + q.c1; f1 = f1 * d + f;
-  return sg * f1 > 0.f && f2 > 0.f && sg * f3 > 0.f;
-}
-
-// Both extreme roots from the given starts.  A step of s leaves an error of order s^3, so the
-// step below 5e-4 is the last one.
+// Both extreme roots from the starts hi and lo, which must lie outside them.  A step of s leaves an
+// error of order s^3, so the step below 5e-4 is the last one.
 __device__ __forceinline__ void laguerre_pair(const FastQuartic &q, float &hi, float &lo)
 {
 #pragma unroll 1
