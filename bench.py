@@ -100,16 +100,16 @@ CFL = 0.3
 # utilisation that bounds the lean HLLD sweeps.  They come from separate captures, not from
 # the run that prints them.
 NCU_TRAFFIC_PER_UNIT = {("update", "plm", "hlld", "lean"): 69.7,    # a first-stage CT launch
-                        # a first-stage x sweep's DRAM bytes per zone, 104.1 against its 80
-                        # algorithmic, applied as that 1.301 ratio to the mean of the three sweeps
-                        # (86.7 B); for WENO5 a y sweep's 82.2 against 80
-                        ("flux", "plm", "hlld", "lean"): 112.8,
-                        ("flux", "weno5", "hlld", "lean"): 89.1}
+                        # a first-stage x sweep's DRAM bytes per zone, 103.9 against its 80
+                        # algorithmic, applied as that 1.299 ratio to the mean of the three sweeps
+                        # (86.7 B); for WENO5 a y sweep's 82.1 against 80
+                        ("flux", "plm", "hlld", "lean"): 112.6,
+                        ("flux", "weno5", "hlld", "lean"): 89.0}
 NCU_LIMITER = {
-    ("flux", "plm", "hlld", "lean"): {"issue_active": 0.683, "fma_pipe": 0.382, "xu_pipe": 0.197,
-                                      "dram_throughput": 0.148},
-    ("flux", "weno5", "hlld", "lean"): {"issue_active": 0.619, "fma_pipe": 0.380, "xu_pipe": 0.244,
-                                        "dram_throughput": 0.090},
+    ("flux", "plm", "hlld", "lean"): {"issue_active": 0.691, "fma_pipe": 0.392, "xu_pipe": 0.205,
+                                      "dram_throughput": 0.147},
+    ("flux", "weno5", "hlld", "lean"): {"issue_active": 0.630, "fma_pipe": 0.390, "xu_pipe": 0.252,
+                                        "dram_throughput": 0.092},
 }
 
 

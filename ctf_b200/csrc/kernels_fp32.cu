@@ -12,8 +12,8 @@
 #ifndef MGPU_HLLD_MINB
 #define MGPU_HLLD_MINB 6
 #endif
-// zone c2p at 8 blocks, 64 registers (the FP64 state is live only through one or two Newton
-// steps): 160^3 lean c2p per RK3 step 0.68 / 0.62 / 0.56 ms at 5 / 6 / 8 blocks
+// zone c2p at 8 blocks, 64 registers (the FP64 state is live only through two or three Newton
+// steps): 160^3 lean c2p per RK3 step 0.74 / 0.68 / 0.64 / 0.62 ms at 5 / 6 / 7 / 8 blocks
 #ifdef MGPU_C2P_MINB_OVERRIDE
 #define MGPU_C2P_MINB MGPU_C2P_MINB_OVERRIDE
 #else

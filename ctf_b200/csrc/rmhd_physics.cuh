@@ -4,10 +4,13 @@
 //
 // Everything is templated on the bulk arithmetic type T.  With T = double and the
 // translation unit compiled with --fmad=false, every expression is evaluated in the same
-// IEEE operation order as the reference's gcc build, so the plain FP64 path reproduces the
-// reference bit for bit except where CUDA's pow/acos/cos/sin differ from glibc by an ulp
-// (the quartic only).  With T = float the same algorithms run in FP32 with tolerances
-// rescaled to FP32 resolution (RmhdTol<float>); the c2p Newton polish stays FP64 always.
+// IEEE operation order as the reference's gcc build (quotients by a shared divisor through its
+// reciprocal, with the same bits), so the plain FP64 path reproduces the reference bit for bit
+// except in two places: CUDA's pow/acos/cos/sin differ from glibc by an ulp (the quartic only),
+// and the root of HLLD's eq. 48 is reached by fewer evaluations from a start that is inverted in
+// FP32 (hlld_solve: the same root and the same fallbacks, the flux to rounding, 1e-12 at worst).
+// With T = float the same algorithms run in FP32 with tolerances rescaled to FP32 resolution
+// (RmhdTol<float>); the c2p starts in FP32 and ends in FP64, on the FP64 path's bound.
 //
 // Reference sources restated here (paths within the reference project):
 //   EOS          Mara/eos.cpp:13-29                    P->U         Mara/rmhd.cpp:177-207
@@ -399,7 +402,7 @@ __device__ __forceinline__ void flux_and_eigenvalues(T gamma, const T *U, const 
   quartic_extreme_roots<T>(A4, A3, A2, A1, A0, ap, am);
 }
 
-// ---- c2p: Newton solvers and the four-attempt ladder (FP64 always) --------------------------
+// ---- c2p: Newton solvers and the four-attempt ladder (FP64; the FP32 bulk path starts in FP32) ----
 struct C2PState {
   double D, Tau, S2, B2, BS, BS2, gamma, gamf, pfloor;
   double Sxyz[3], Bxyz[3];
@@ -1175,7 +1178,7 @@ static __device__ __noinline__ HllcOut<T> riemann_hllc_fallback(int dim, T gamma
   return o;
 }
 
-// ---- HLLD (Mignone, Ugliano & Bodo 2009; Mara/riemann_hlld-rmhd.cpp) -------------------------
+// ---- columns in shared memory ------------------------------------------------------------------
 // A thread's column of an array of shared memory (entry i at p[i * stride]): the stride is the
 // block's width, so a warp's accesses to one entry are conflict-free.
 template <class T> struct Column {
