@@ -524,14 +524,15 @@ static int transfer(mgpu_solver *h, double *host, const void *dev_in, void *dev_
   // a pageable buffer goes through two pinned chunk slots (xfer_host), chunk by chunk: the threaded
   // host copy of one chunk overlaps the DMA copy and conversion of the other.  The driver moves
   // pageable memory at 13 to 20 GB/s; upload / download, as they are against staged: 8 MB
-  // 0.52 / 0.57 -> 0.36 / 0.34 ms, 22 MB 1.31 / 1.48 -> 1.11 / 1.06, 64 MB 4.4 / 5.1 -> 2.5 / 2.3;
-  // 4 to 6 MB 0.30 to 0.42 -> 0.2 to 0.6, so those go as they are.  Below 64 MB making the slots
-  // costs as much as some eight transfers of 22 MB gain (25 of 8 MB, two of 64 MB), so a solver's
-  // first eight go as they are: a solver that is filled, advanced and read once does not pay for
-  // slots that it hardly uses.
+  // 0.52 / 0.57 -> 0.36 / 0.34 ms, 22 MB 1.31 / 1.48 -> 1.11 / 1.06, 64 MB 4.4 / 5.1 -> 2.5 / 2.3.
+  // In loops of Mara.advance on a pageable FP64 box the call gains down to 4 MB (36^3, 4.7 MB:
+  // 1.40 -> 1.33 ms; 42^3, 7.1 MB: 1.97 -> 1.60).  Below 64 MB making the slots costs as much as
+  // some eight transfers of 22 MB gain (25 of 8 MB, two of 64 MB), so a solver's first eight go as
+  // they are: a solver that is filled, advanced and read once does not pay for slots that it
+  // hardly uses.
   bool staged = false;
   const size_t bytes = (size_t) (nz - zbeg) * 8 * sizeof(double);
-  if (bytes >= (size_t(8) << 20)) {
+  if (bytes >= (size_t(4) << 20)) {
     cudaPointerAttributes pa{};
     const bool pinned = cudaPointerGetAttributes(&pa, host + zbeg * 8) == cudaSuccess && pa.type == cudaMemoryTypeHost;
     cudaGetLastError();   // an unregistered pointer may leave an error behind

@@ -1,4 +1,4 @@
-"""Whole-array transfers of pageable buffers between 8 and 64 MB, which go as they are for a
+"""Whole-array transfers of pageable buffers between 4 and 64 MB, which go as they are for a
 solver's first eight and through pinned chunk slots from then on: every one brings the same bytes."""
 import numpy as np
 import pytest
@@ -9,8 +9,8 @@ from ctf_b200.mara import Scheme, Solver
 pytestmark = pytest.mark.gpu
 
 
-# 37^3 guarded zones and 41 x 42 x 39: below 8 MB; 51 x 52 x 50: just above, five chunks with a short
-# last one; 64^3 guarded zones: whole chunks only
+# 37^3 guarded zones: below 4 MB; 41 x 42 x 39: just above, three chunks with a short last one;
+# 51 x 52 x 50: five; 64^3 guarded zones: whole chunks only
 @pytest.mark.parametrize("n", [(31, 31, 31), (35, 36, 33), (45, 46, 44), (58, 58, 58)])
 def test_repeated_pageable_transfers_bring_the_same_bytes(n):
     P = ics.turbulence_box(n, seed=3)
