@@ -301,8 +301,8 @@ def test_fp32_speeds_down_to_the_coldest_gas(lib):
 @pytest.mark.parametrize("angle,jump,dv", [(0.01, 0.1, 0.02), (0.05, 0.02, 0.02), (0.02, 0.05, 0.01)])
 def test_fp32_outer_speeds_where_fast_and_slow_meet(lib, angle, jump, dv):
     """Faces with the field nearly along the sweep and Alfven and sound speeds nearly equal: the
-    fast and slow roots of a side almost coincide, and the other side's correction must not
-    start its iteration between them.  Rounding of 1e-7 in the coefficients moves a double
+    fast and slow roots of a side almost coincide, and each side's iteration must end at its
+    own fast root, wherever it is started from.  Rounding of 1e-7 in the coefficients moves a double
     root by the square root of that: 1e-3 allows for a condition of ten."""
     rng = np.random.default_rng(11)
     n = 4000
